@@ -420,6 +420,7 @@ int job_launch_centroids(mc_job *j, const uint32_t *keys2, uint64_t extra, bool 
     ca.w = j->w.p;
     ca.centers = j->Cw.p;
     ca.nan_flag = j->flag.p;
+    ca.keep_bands = true;  // j->sort sorts rows of j->M only
     MC_CUDA_TRY(cudaMemsetAsync(j->flag.p, 0, sizeof(int), st));
     return launch_centroids(ca, j->sort, st, presorted);
 }

@@ -547,24 +547,6 @@ int launch_sort_by_key(const uint32_t *keys, const uint32_t *keys2, uint64_t n, 
 // chunk_start[c] = exclusive scan of the chunk counts (computed on device); a grid of
 // ceil(n/ch)+k CTAs maps its chunk id by binary search, extra CTAs exit.
 // ------------------------------------------------------------------------------------
-__device__ inline uint32_t find_bucket(const uint64_t *chunk_start, uint32_t k, uint64_t q) {
-    // largest c with chunk_start[c] <= q (chunk_start has k+1 entries, nondecreasing)
-    uint32_t lo = 0, hi = k;  // invariant: chunk_start[lo] <= q < chunk_start[hi]
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (chunk_start[mid] <= q) lo = mid; else hi = mid;
-    }
-    return lo;
-}
-
-__device__ inline void two_sum_add(float &s, float &e, float x) {
-    const float t = __fadd_rn(s, x);
-    const float bp = __fsub_rn(t, s);
-    const float err = __fadd_rn(__fsub_rn(s, __fsub_rn(t, bp)), __fsub_rn(x, bp));
-    s = t;
-    e = __fadd_rn(e, err);
-}
-
 // dense: one CTA per chunk (at most kDenseChunk rows of one cluster), threads over
 // columns, rows sequential.  The chunk's row ids are staged in shared memory and each
 // thread loads 8 rows' values ahead of its sequential sum, so the loads overlap.
@@ -802,76 +784,6 @@ __global__ void k_centroid_chunks_csr_short(const float *__restrict__ vals, cons
     }
 }
 
-// The same sums for short rows and narrow bands (d <= 2048): the chunk's rows are taken
-// kCsrTileRows at a time and scattered into a dense [rows][512 columns] tile in shared
-// memory (rows in parallel, one warp each); then each thread walks its column down the tile
-// in row order.  A column's additions are the same as in k_centroid_chunks_csr_short (every
-// stored value of the column, rows ascending; a zero added by TwoSum or by the weighted fma
-// leaves the sum unchanged, so empty tile cells are skipped), so the partials are
-// bit-identical, but the rows of a batch are loaded concurrently instead of one dependent
-// round trip per row.
-constexpr int kCsrTileRows = 32, kCsrTileBand = 512;
-
-__global__ void __launch_bounds__(kCsrTileBand) k_centroid_chunks_csr_tile(
-    const float *__restrict__ vals, const uint32_t *__restrict__ idx, const uint64_t *__restrict__ indptr, uint64_t d,
-    const uint32_t *__restrict__ perm, const uint64_t *__restrict__ bucket_start,
-    const uint64_t *__restrict__ bucket_count, const uint64_t *__restrict__ chunk_start, uint32_t k, uint64_t ch,
-    const double *__restrict__ w, double *partial, double *partial_w) {
-    extern __shared__ __align__(16) float tile[];  // [kCsrTileRows][kCsrTileBand]
-    __shared__ uint64_t rb[kCsrTileRows], re[kCsrTileRows];
-    __shared__ double rw[kCsrTileRows];
-    const uint64_t q = blockIdx.x;
-    if (q >= chunk_start[k]) return;
-    const uint32_t c = find_bucket(chunk_start, k, q);
-    const uint64_t local = q - chunk_start[c];
-    const uint64_t r0 = local * ch, r1 = umin64(bucket_count[c], r0 + ch);
-    const uint32_t *rows = perm + bucket_start[c];
-    const uint64_t j0 = uint64_t(blockIdx.y) * kCsrTileBand, j1 = umin64(d, j0 + kCsrTileBand);
-    const int t = threadIdx.x, lane = t & 31, wp = t >> 5;
-    constexpr int NW = kCsrTileBand / 32;
-    const bool weighted = w != nullptr;
-    for (int e = t; e < kCsrTileRows * kCsrTileBand; e += kCsrTileBand) tile[e] = 0.f;
-    const uint64_t j = j0 + uint64_t(t);
-    float s = 0.f, er = 0.f;
-    double acc = 0.0, wq = 0.0;
-    for (uint64_t b0 = r0; b0 < r1; b0 += kCsrTileRows) {
-        const int nb = int(umin64(kCsrTileRows, r1 - b0));
-        if (t < nb) {
-            const uint32_t row = rows[b0 + t];
-            rb[t] = indptr[row];
-            re[t] = indptr[row + 1];
-            if (weighted) rw[t] = w[row];
-        }
-        __syncthreads();
-        for (int rr = wp; rr < nb; rr += NW)
-            for (uint64_t p = rb[rr] + lane; p < re[rr]; p += 32) {
-                const uint32_t col = idx[p];
-                if (col >= j0 && col < j1) tile[rr * kCsrTileBand + int(col - j0)] = vals[p];
-            }
-        __syncthreads();
-        if (j < j1) {
-            for (int rr = 0; rr < nb; ++rr) {
-                const float v = tile[rr * kCsrTileBand + t];
-                if (v != 0.f) {
-                    if (weighted) acc = fma(rw[rr], double(v), acc);
-                    else two_sum_add(s, er, v);
-                }
-            }
-        }
-        if (weighted && t == 0 && blockIdx.y == 0)
-            for (int rr = 0; rr < nb; ++rr) wq = wq + rw[rr];
-        __syncthreads();
-        for (int rr = wp; rr < nb; rr += NW)
-            for (uint64_t p = rb[rr] + lane; p < re[rr]; p += 32) {
-                const uint32_t col = idx[p];
-                if (col >= j0 && col < j1) tile[rr * kCsrTileBand + int(col - j0)] = 0.f;
-            }
-        __syncthreads();
-    }
-    if (j < j1) partial[q * d + j] = weighted ? acc : double(s) + double(er);
-    if (weighted && t == 0 && blockIdx.y == 0) partial_w[q] = wq;
-}
-
 // finalize: per (bucket, column): FP64 sum of chunk partials in order, divide, round.
 // Buckets with one row copy the row (here for dense rows X; CSR rows in
 // k_centroid_singletons_csr); empty buckets keep the old center.
@@ -935,25 +847,16 @@ int launch_centroids(const CentroidArgs &a, SortWork &w, cudaStream_t st, bool p
                                                                      w.bucket_count.p, w.chunk_start.p, k, ch, a.w,
                                                                      w.partial.p, w.partial_w.p), note_launch();
     } else {
-        const uint64_t band = a.w ? 12288 : 24576;  // 96 KB (double) or 192 KB (two floats)
-        const uint64_t bw = band < d ? band : d;
-        const size_t smem = a.w ? bw * sizeof(double) : 2 * bw * sizeof(float);
-        const unsigned nb = unsigned((d + band - 1) / band);
-        // always the largest band's size: a per-call value could be lowered by another host
-        // thread between this call's set and its launch
-        // rows of 32 or more nonzeros on average: the register-pipelined kernel
-        if (a.nnz < 32 * n && d <= 4 * uint64_t(kCsrTileBand)) {
-            // short rows over at most four 512-column bands: rows of a batch scattered into a
-            // dense shared-memory tile, columns walked in row order
-            const size_t tsm = size_t(kCsrTileRows) * kCsrTileBand * sizeof(float);
-            MC_CUDA_TRY(cudaFuncSetAttribute(k_centroid_chunks_csr_tile, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             int(tsm)));
-            k_centroid_chunks_csr_tile<<<dim3(unsigned(max_chunks), unsigned((d + kCsrTileBand - 1) / kCsrTileBand)),
-                                         kCsrTileBand, tsm, st>>>(a.vals, a.idx, a.indptr, d, w.perm.p,
-                                                                  w.bucket_start.p, w.bucket_count.p,
-                                                                  w.chunk_start.p, k, ch, a.w, w.partial.p,
-                                                                  w.partial_w.p), note_launch();
-        } else {
+        bool done = false;
+        MC_TRY(launch_centroid_chunks_csr(a, w, max_chunks, ch, st, &done));
+        if (!done) {
+            const uint64_t band = a.w ? 12288 : 24576;  // 96 KB (double) or 192 KB (two floats)
+            const uint64_t bw = band < d ? band : d;
+            const size_t smem = a.w ? bw * sizeof(double) : 2 * bw * sizeof(float);
+            const unsigned nb = unsigned((d + band - 1) / band);
+            // always the largest band's size: a per-call value could be lowered by another
+            // host thread between this call's set and its launch
+            // rows of 32 or more nonzeros on average: the register-pipelined kernel
             auto kern = (a.nnz >= 32 * n) ? k_centroid_chunks_csr : k_centroid_chunks_csr_short;
             MC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              int(2 * 24576 * sizeof(float))));

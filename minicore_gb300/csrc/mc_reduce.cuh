@@ -15,6 +15,8 @@ struct SortWork {
     DBuf<uint64_t> chunk_start;   // [k+1]
     DBuf<double> partial;         // [chunks][d]
     DBuf<double> partial_w;       // [chunks]
+    DBuf<uint32_t> bands;         // CSR centroid sums: [n][bands + 1] row offsets of the column bands
+    bool bands_ready = false;     // bands holds the offsets of the owning job's matrix
 };
 
 struct CentroidArgs {
@@ -32,10 +34,32 @@ struct CentroidArgs {
     const double *w = nullptr;                // optional row weights
     float *centers = nullptr;                 // [k][d], updated in place
     int *nan_flag = nullptr;
+    bool keep_bands = false;                  // CSR: the SortWork belongs to this matrix (keep its bands)
 };
+
+__device__ inline uint32_t find_bucket(const uint64_t *chunk_start, uint32_t k, uint64_t q) {
+    // largest c with chunk_start[c] <= q (chunk_start has k+1 entries, nondecreasing)
+    uint32_t lo = 0, hi = k;  // invariant: chunk_start[lo] <= q < chunk_start[hi]
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (chunk_start[mid] <= q) lo = mid; else hi = mid;
+    }
+    return lo;
+}
+
+__device__ inline void two_sum_add(float &s, float &e, float x) {
+    const float t = __fadd_rn(s, x);
+    const float bp = __fsub_rn(t, s);
+    const float err = __fadd_rn(__fsub_rn(s, __fsub_rn(t, bp)), __fsub_rn(x, bp));
+    s = t;
+    e = __fadd_rn(e, err);
+}
 
 int launch_sort_by_key(const uint32_t *keys, const uint32_t *keys2, uint64_t n, uint32_t k, SortWork &w,
                        cudaStream_t st);
+// chunk partials over CSR rows (mc_centroid_csr.cu); *done = false: not covered there
+int launch_centroid_chunks_csr(const CentroidArgs &a, SortWork &w, uint64_t max_chunks, uint64_t ch, cudaStream_t st,
+                               bool *done);
 // presorted: w already holds the counting sort of a.keys (no second membership)
 int launch_centroids(const CentroidArgs &a, SortWork &w, cudaStream_t st, bool presorted = false);
 
