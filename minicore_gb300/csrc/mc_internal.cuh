@@ -132,6 +132,13 @@ __host__ __device__ inline uint64_t det_leaves(uint64_t n) {
 // doubles of scratch that launch_det_sum / launch_det_draw need (the tree, heap layout)
 __host__ __device__ inline uint64_t det_tmp_size(uint64_t n) { return 2 * det_leaves(n); }
 
+// pairwise sum of 32 consecutive elements held one per lane; the result is in lane 0
+__device__ __forceinline__ double lane_pairwise32(double v) {
+#pragma unroll
+    for (int sft = 1; sft < 32; sft <<= 1) v = v + __shfl_down_sync(0xffffffffu, v, sft);
+    return v;
+}
+
 // value sources for det sums
 enum DetSrc : int {
     DET_F64 = 0,        // x[i]
@@ -241,6 +248,9 @@ __host__ __device__ inline uint64_t umin64(uint64_t a, uint64_t b) { return a < 
 int launch_det_sum(const DetInput &in, double *chunk_tmp, double *out, cudaStream_t st);
 int launch_det_draw(const DetInput &in, double *chunk_tmp, const double *u_dev, double u_host, int use_dev_u,
                     const double *fallback_vals, uint64_t *out_idx, cudaStream_t st);
+// the same draw from the sums of 32-element blocks (n > 0); ticket: a zero that it leaves zero
+int launch_det_draw_blocks(const DetInput &in, const double *blk, double *chunk_tmp, unsigned *ticket,
+                           const double *u_dev, const double *fallback_vals, uint64_t *out_idx, cudaStream_t st);
 
 // dense + CSR row statistics
 int launch_row_sums_dense(const float *X, uint64_t n, uint64_t d, double *rowsum, float *rownorm, cudaStream_t st);

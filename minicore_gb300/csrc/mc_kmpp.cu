@@ -74,6 +74,16 @@ __device__ __forceinline__ bool kp_prune(const KmppArgs &a, uint64_t i, double c
     return t * t * (1.0 - g) * (1.0 - 0x1p-48) >= cur;
 }
 
+// The block sum of the warp's 32 rows (lane l: row i = 32b + l and its distance v after the
+// update), written where a row changed.  Every lane of the warp calls it.
+__device__ __forceinline__ void kp_block_out(const KmppArgs &a, uint64_t i, double v, bool changed) {
+    if (!a.blk || !__any_sync(0xffffffffu, changed)) return;
+    if (i >= a.n) v = 0.0;
+    else if (a.w) v = v * a.w[i];
+    v = lane_pairwise32(v);
+    if ((threadIdx.x & 31) == 0) a.blk[i >> 5] = v;
+}
+
 // per round: a lower bound of ||X[new center] - X[center a]|| for every earlier center
 // a < round (one warp each; FP64 sum of squared differences of the float rows, shrunk by its
 // rounding bound)
@@ -124,30 +134,21 @@ __global__ void k_kmpp_scatter(const KmppArgs a) {
         a.cbuf[a.idx[p]] = a.vals[p];
 }
 
-__global__ void k_kmpp_zero(const KmppArgs a) { a.dist[*a.newc] = 0.0; }
-
-// dense rows: one thread per row; the row and the new center are read with float4 loads
-// in 32-column chunks (16 loads in flight per thread), the reduction stays sequential over
-// the columns (the oracle's order).  Rounds after the first also record the center
-// (center_ids, asn) and zero its distance, so no separate launches are needed.
+// row i's update against center row c (read with float4 loads in 32-column chunks, 16 loads
+// in flight); returns its distance afterwards
 template <int MSR, bool VEC4>
-__global__ void __launch_bounds__(256) k_kmpp_dense(const KmppArgs a, int first) {
-    const uint64_t c = *a.newc;
-    if (!first && blockIdx.x == 0 && threadIdx.x == 0) {
-        a.center_ids[a.round] = uint32_t(c);
-        a.asn[c] = a.round;
-    }
-    const uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
-    if (i >= a.n) return;
+__device__ __forceinline__ double kp_dense_row(const KmppArgs &a, uint64_t i, uint64_t c, int first, bool &changed) {
+    if (i >= a.n) return 0.0;
     double cur = 0.0;
     if (!first) {
         if (i == c) {
             a.dist[i] = 0.0;
-            return;
+            changed = true;
+            return 0.0;
         }
         cur = a.dist[i];
-        if (cur <= 0.0) return;
-        if (MSR == SQRL2 && a.cgap && kp_prune(a, i, cur)) return;
+        if (cur <= 0.0) return cur;
+        if (MSR == SQRL2 && a.cgap && kp_prune(a, i, cur)) return cur;
     }
     PairScalars s = {};
     if (MSR != SQRL2) s = pair_scalars(a.prior, a.prior_sum, a.rowsum[i], a.rowsum[c], a.d);
@@ -184,11 +185,56 @@ __global__ void __launch_bounds__(256) k_kmpp_dense(const KmppArgs a, int first)
     }
     const double v = kp_cost<MSR>(acc);
     if (first) {
-        a.dist[i] = (i == c) ? 0.0 : v;
-    } else if (v < cur) {
+        changed = true;
+        return a.dist[i] = (i == c) ? 0.0 : v;
+    }
+    if (v < cur) {
+        changed = true;
         a.dist[i] = v;
         a.asn[i] = a.round;
+        return v;
     }
+    return cur;
+}
+
+// dense rows: one thread per row; the row and the new center are read with float4 loads
+// in 32-column chunks (16 loads in flight per thread), the reduction stays sequential over
+// the columns (the oracle's order).  Rounds after the first also record the center
+// (center_ids, asn) and zero its distance, so no separate launches are needed.
+template <int MSR, bool VEC4>
+__global__ void __launch_bounds__(256) k_kmpp_dense(const KmppArgs a, int first) {
+    const uint64_t c = *a.newc;
+    if (!first && blockIdx.x == 0 && threadIdx.x == 0) {
+        a.center_ids[a.round] = uint32_t(c);
+        a.asn[c] = a.round;
+    }
+    const uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
+    bool changed = false;
+    const double now = kp_dense_row<MSR, VEC4>(a, i, c, first, changed);
+    kp_block_out(a, i, now, changed);
+}
+
+// CSR rows of a warp (lane l: row my, its new distance v where go): the minimum with the
+// current distance, the center's own row at 0, and the rows' block sum
+__device__ __forceinline__ void kp_csr_row_out(const KmppArgs &a, int first, uint32_t round, uint64_t c, uint64_t my,
+                                               bool go, double v) {
+    double now = 0.0;
+    bool changed = false;
+    if (my < a.n) {
+        if (first || my == c) {
+            now = (my == c) ? 0.0 : v;
+            changed = true;
+        } else {
+            now = a.dist[my];
+            if (go && v < now) {
+                now = v;
+                a.asn[my] = round;
+                changed = true;
+            }
+        }
+        if (changed) a.dist[my] = now;
+    }
+    kp_block_out(a, my, now, changed);
 }
 
 // CSR rows (any measure, any prior): sum over all columns of f(a_j, b0) (b0: transform of a
@@ -239,15 +285,9 @@ __global__ void __launch_bounds__(256) k_kmpp_csr(const KmppArgs a, int first, u
             for (int m = 16; m >= 1; m >>= 1) acc = acc + __shfl_xor_sync(0xffffffffu, acc, m);
             if (lane == r) accm = acc;
         }
-        if (!go) continue;
         double v = kp_cost<MSR>(accm);
         if (MSR == SQRL2 && v < 0.0) v = 0.0;
-        if (first) {
-            a.dist[my] = (my == c) ? 0.0 : v;
-        } else if (v < a.dist[my]) {
-            a.dist[my] = v;
-            a.asn[my] = round;
-        }
+        kp_csr_row_out(a, first, round, c, my, go, v);
     }
 }
 
@@ -469,9 +509,9 @@ __device__ __forceinline__ void kp_nnz_rows(const KmppArgs &a, int first, uint32
                 if (lane == r) accm = acc;
             }
         }
-        if (!go) continue;
-        double v;
-        if (fastm) {
+        double v = 0.0;
+        if (!go) {
+        } else if (fastm) {
             float key;
             if (MSR == SQRL2) {
                 double t = K0 + double(accm);
@@ -496,12 +536,7 @@ __device__ __forceinline__ void kp_nnz_rows(const KmppArgs &a, int first, uint32
             v = kp_cost<MSR>(accm);
             if (MSR == SQRL2 && v < 0.0) v = 0.0;
         }
-        if (first) {
-            a.dist[my] = (my == c) ? 0.0 : v;
-        } else if (v < a.dist[my]) {
-            a.dist[my] = v;
-            a.asn[my] = round;
-        }
+        kp_csr_row_out(a, first, round, c, my, go, v);
     }
 }
 
@@ -530,7 +565,6 @@ __global__ void __launch_bounds__(1024) k_kmpp_csr_fused(const KmppArgs a, int f
     if (blockIdx.x == 0 && tid == 0) {
         a.center_ids[round] = uint32_t(c);
         a.asn[c] = round;
-        if (!first) a.dist[c] = 0.0;
     }
     __syncthreads();
     const float pv = float(a.prior);
@@ -587,11 +621,12 @@ __global__ void __launch_bounds__(128) k_kmpp_dense_staged(const KmppArgs a, int
     const int t = threadIdx.x;
     const uint64_t row0 = uint64_t(blockIdx.x) * 128;
     const uint64_t i = row0 + t;
-    bool active = i < a.n;
+    bool active = i < a.n, changed = false;
     double cur = 0.0;
     if (active && !first) {
         if (i == c) {
             a.dist[i] = 0.0;
+            changed = true;
             active = false;
         } else {
             cur = a.dist[i];
@@ -602,7 +637,10 @@ __global__ void __launch_bounds__(128) k_kmpp_dense_staged(const KmppArgs a, int
     // rows that need no distance are not staged; a CTA with none left stops here
     __shared__ unsigned char act_s[128];
     act_s[t] = active ? 1 : 0;
-    if (!__syncthreads_or(active ? 1 : 0)) return;
+    if (!__syncthreads_or(active ? 1 : 0)) {
+        kp_block_out(a, i, cur, changed);
+        return;
+    }
     PairScalars s = {};
     if (active && MSR != SQRL2) s = pair_scalars(a.prior, a.prior_sum, a.rowsum[i], a.rowsum[c], a.d);
     const uint64_t d = a.d;
@@ -643,14 +681,18 @@ __global__ void __launch_bounds__(128) k_kmpp_dense_staged(const KmppArgs a, int
         }
         __syncthreads();  // buffer buf is restaged two chunks later
     }
-    if (!active) return;
-    const double v = kp_cost<MSR>(acc);
-    if (first) {
-        a.dist[i] = (i == c) ? 0.0 : v;
-    } else if (v < cur) {
-        a.dist[i] = v;
-        a.asn[i] = a.round;
+    if (active) {
+        const double v = kp_cost<MSR>(acc);
+        if (first) {
+            cur = a.dist[i] = (i == c) ? 0.0 : v;
+            changed = true;
+        } else if (v < cur) {
+            cur = a.dist[i] = v;
+            a.asn[i] = a.round;
+            changed = true;
+        }
     }
+    kp_block_out(a, i, cur, changed);
 }
 
 // The same with persistent CTAs: each of sms x 4 CTAs walks its row tiles (stride gridDim)
@@ -671,14 +713,16 @@ __global__ void __launch_bounds__(128) k_kmpp_dense_persist(const KmppArgs a, in
     }
     const int t = threadIdx.x;
     const uint64_t d = a.d, nchunk = (d + 31) / 32, ntiles = (a.n + 127) / 128;
-    auto row_state = [&](uint64_t m, bool &act, double &cur, PairScalars &ps) {
+    auto row_state = [&](uint64_t m, bool &act, double &cur, PairScalars &ps, bool &chg) {
         const uint64_t i = m * 128 + uint64_t(t);
         act = i < a.n;
+        chg = false;
         cur = 0.0;
         ps = PairScalars{0.f, 0.f, 0.f, 0.f, 0.f};
         if (act && !first) {
             if (i == c) {
                 a.dist[i] = 0.0;
+                chg = true;
                 act = false;
             } else {
                 cur = a.dist[i];
@@ -704,10 +748,10 @@ __global__ void __launch_bounds__(128) k_kmpp_dense_persist(const KmppArgs a, in
     };
     uint64_t m = blockIdx.x;
     if (m >= ntiles) return;
-    bool active;
+    bool active, changed;
     double cur;
     PairScalars ps;
-    row_state(m, active, cur, ps);
+    row_state(m, active, cur, ps, changed);
     int ab = 0, buf = 0;
     act_s[ab][t] = active ? 1 : 0;
     __syncthreads();
@@ -718,13 +762,13 @@ __global__ void __launch_bounds__(128) k_kmpp_dense_persist(const KmppArgs a, in
             const bool last = ci + 1 == nchunk;
             const uint64_t mn = m + gridDim.x;
             const bool have_next = !last || mn < ntiles;
-            bool act2 = false;
+            bool act2 = false, chg2 = false;
             double cur2 = 0.0;
             PairScalars ps2 = PairScalars{0.f, 0.f, 0.f, 0.f, 0.f};
             if (!last) {
                 stage(m, ci + 1, buf ^ 1, ab);
             } else if (have_next) {
-                row_state(mn, act2, cur2, ps2);
+                row_state(mn, act2, cur2, ps2, chg2);
                 act_s[ab ^ 1][t] = act2 ? 1 : 0;
                 __syncthreads();
                 stage(mn, 0, buf ^ 1, ab ^ 1);
@@ -744,19 +788,23 @@ __global__ void __launch_bounds__(128) k_kmpp_dense_persist(const KmppArgs a, in
             __syncthreads();  // buffer buf is restaged in the next iteration
             buf ^= 1;
             if (last) {
+                const uint64_t i = m * 128 + uint64_t(t);
                 if (active) {
-                    const uint64_t i = m * 128 + uint64_t(t);
                     const double v = kp_cost<MSR>(acc);
                     if (first) {
-                        a.dist[i] = (i == c) ? 0.0 : v;
+                        cur = a.dist[i] = (i == c) ? 0.0 : v;
+                        changed = true;
                     } else if (v < cur) {
-                        a.dist[i] = v;
+                        cur = a.dist[i] = v;
                         a.asn[i] = a.round;
+                        changed = true;
                     }
                 }
+                kp_block_out(a, i, cur, changed);
                 if (!have_next) return;
                 m = mn;
                 active = act2;
+                changed = chg2;
                 cur = cur2;
                 ps = ps2;
                 ab ^= 1;
@@ -1131,8 +1179,9 @@ static int run_kmeanspp_cluster(const KmppArgs &a, const double *u_dev, cudaStre
 // where Sb = ||xb - c||^2 lies in [A / (1 + g), A / (1 - g)], and v >= S (1 - g), with
 // g = (d + 2) 2^-24 / (1 - (d + 2) 2^-24) (the bound of an FP32 sum of d squared
 // differences).  k_kmpp_screen evaluates that lower bound of v in FP32 with every rounding
-// directed down (the subtracted terms up) and lists the rows where it does not exceed
-// dist[i]; k_kmpp_exact_list then runs the update's own arithmetic on those rows only.
+// directed down (the subtracted terms up); where it does not exceed dist[i] the row's thread
+// runs the update's own arithmetic at once (a separate pass over a list of those rows took
+// 12 us, and the block sums of the changed rows would have needed one more).
 // Every other row keeps its distance and assignment, as the update would leave them, so the
 // results are bit-identical to the unscreened rounds, and a round reads the 2-byte copy plus
 // the listed rows' FP32 values instead of every FP32 value.
@@ -1142,8 +1191,6 @@ struct ScreenArgs {
     const float *rn2;      // [n] FP32 squared row norms (sequential fmaf)
     float norm_up;         // (1 + (d + 4) 2^-24) rounded up: covers the error of sqrt(rn2)
     float one_m_g, one_p_2g;  // 1 - g rounded down, 1 + 2 g rounded up
-    uint32_t *list;        // rows for the exact update
-    unsigned *count;
 };
 
 // One row per thread, 128 rows per CTA: the rows' BF16 values staged in shared memory by
@@ -1154,7 +1201,7 @@ __global__ void __launch_bounds__(128) k_kmpp_screen(const KmppArgs a, const Scr
     __shared__ __align__(16) uint4 xs[128 * P];
     __shared__ __align__(16) float cs[8 * G];
     const uint64_t c = *a.newc;
-    const int t = threadIdx.x, lane = t & 31;
+    const int t = threadIdx.x;
     if (blockIdx.x == 0 && t == 0) {
         a.center_ids[a.round] = uint32_t(c);
         a.asn[c] = a.round;
@@ -1214,52 +1261,40 @@ __global__ void __launch_bounds__(128) k_kmpp_screen(const KmppArgs a, const Scr
             need = !(vb > cb) || !(A <= 3.402823466e+38f) || !(xn <= 3.402823466e+38f) || !(vlo <= 3.402823466e+38f);
         }
     }
-    const unsigned nb = __ballot_sync(0xffffffffu, need);
-    if (nb) {
-        unsigned base = 0;
-        if (lane == 0) base = atomicAdd(sa.count, unsigned(__popc(nb)));
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (need) sa.list[base + __popc(nb & ((1u << lane) - 1u))] = uint32_t(i);
-    }
-}
-
-// The update's arithmetic (k_kmpp_dense) on the listed rows: the sequential fmaf sum over the
-// columns, replaced only when below the current distance.
-__global__ void __launch_bounds__(256) k_kmpp_exact_list(const KmppArgs a, const uint32_t *__restrict__ list,
-                                                         const unsigned *__restrict__ count) {
-    extern __shared__ __align__(16) float csm[];  // the new center's row
-    const uint64_t c = *a.newc;
-    for (uint64_t j = threadIdx.x; j < a.d; j += blockDim.x) csm[j] = a.X[c * a.d + j];
-    __syncthreads();
-    const unsigned cnt = *count;
-    const PairScalars ps = {};
-    for (uint64_t e = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; e < cnt; e += gridDim.x * uint64_t(blockDim.x)) {
-        const uint64_t i = list[e];
+    double now = __longlong_as_double((long long)cb);
+    bool changed = i == c;
+    if (changed) now = 0.0;
+    if (need) {
+        // the update's arithmetic (k_kmpp_dense) on the FP32 row: the sequential fmaf sum over
+        // the columns, 32 columns' loads in flight, replaced only when below the distance
         const float4 *xr = reinterpret_cast<const float4 *>(a.X + i * a.d);
+        const PairScalars ps = {};
         float acc = 0.f;
-        // 32 columns at a time: their eight loads in flight together (d is a multiple of 16)
-        for (uint64_t j0 = 0; j0 < a.d / 4; j0 += 8) {
+        constexpr int D4 = 2 * G;  // float4 per row
+#pragma unroll
+        for (int j0 = 0; j0 < D4; j0 += 8) {
             float4 x[8];
-            const uint64_t m = a.d / 4 - j0 < 8 ? a.d / 4 - j0 : 8;
 #pragma unroll
-            for (int u = 0; u < 8; ++u) x[u] = uint64_t(u) < m ? xr[j0 + u] : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int u = 0; u < 8; ++u)
+                if (j0 + u < D4) x[u] = xr[j0 + u];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                if (uint64_t(u) < m) {
-                    const float *cc = csm + 4 * (j0 + u);
+            for (int u = 0; u < 8; ++u)
+                if (j0 + u < D4) {
+                    const float *cc = cs + 4 * (j0 + u);
                     kp_elem<SQRL2>(acc, cc[0], x[u].x, ps);
                     kp_elem<SQRL2>(acc, cc[1], x[u].y, ps);
                     kp_elem<SQRL2>(acc, cc[2], x[u].z, ps);
                     kp_elem<SQRL2>(acc, cc[3], x[u].w, ps);
                 }
-            }
         }
         const double v = kp_cost<SQRL2>(acc);
-        if (v < a.dist[i]) {
-            a.dist[i] = v;
+        if (v < now) {
+            now = a.dist[i] = v;
             a.asn[i] = a.round;
+            changed = true;
         }
     }
+    kp_block_out(a, i, now, changed);
 }
 
 // the screened rounds apply: dense SQRL2, d = 8 G with G in {2, 4, 8, 16} (a CTA's staged
@@ -1270,10 +1305,9 @@ static bool kmpp_screen_ok(const KmppArgs &a) {
            (reinterpret_cast<uintptr_t>(a.X) & 15) == 0;
 }
 
-static int screened_round(const KmppArgs &a, uint32_t round, const ScreenArgs &sa, int sms, cudaStream_t st) {
+static int screened_round(const KmppArgs &a, uint32_t round, const ScreenArgs &sa, cudaStream_t st) {
     KmppArgs b = a;
     b.round = round;
-    MC_CUDA_TRY(cudaMemsetAsync(sa.count, 0, sizeof(unsigned), st));
     const unsigned grid = unsigned((a.n + 127) / 128);
     switch (a.d / 8) {
         case 2: k_kmpp_screen<2><<<grid, 128, 0, st>>>(b, sa), note_launch(); break;
@@ -1281,9 +1315,6 @@ static int screened_round(const KmppArgs &a, uint32_t round, const ScreenArgs &s
         case 8: k_kmpp_screen<8><<<grid, 128, 0, st>>>(b, sa), note_launch(); break;
         default: k_kmpp_screen<16><<<grid, 128, 0, st>>>(b, sa), note_launch(); break;
     }
-    // few rows are listed after the first rounds: a small grid (each CTA stages the center)
-    k_kmpp_exact_list<<<unsigned(umin64((a.n + 255) / 256, uint64_t(sms) * 2)), 256, a.d * sizeof(float), st>>>(
-        b, sa.list, sa.count), note_launch();
     MC_CUDA_TRY(cudaGetLastError());
     return MC_OK;
 }
@@ -1324,6 +1355,12 @@ static int run_kmeanspp_launches(const KmppArgs &a0, const double *u_dev, double
                                  cudaStream_t st, bool prune_ok, bool screen_ok) {
     KmppArgs a = a0;
     a.cgap = nullptr;
+    DBuf<double> blk;  // sums of 32 rows' distances, which the draws start from
+    DBuf<unsigned> ticket;
+    MC_TRY(blk.alloc((a.n + 31) / 32, st));
+    MC_TRY(ticket.alloc(1, st));
+    MC_CUDA_TRY(cudaMemsetAsync(ticket.p, 0, sizeof(unsigned), st));
+    a.blk = blk.p;
     const unsigned tb = 256, tg = unsigned(umin64((a.d + tb - 1) / tb, 1024));
     MC_CUDA_TRY(cudaMemsetAsync(a.asn, 0, a.n * sizeof(uint32_t), st));
     k_kmpp_first<<<1, 1, 0, st>>>(u_dev, a.n, a.newc, a.center_ids), note_launch();
@@ -1345,14 +1382,10 @@ static int run_kmeanspp_launches(const KmppArgs &a0, const double *u_dev, double
     const bool screen = screen_ok && !prune && kmpp_screen_ok(a) && a.k > 1;
     DBuf<uint4> xb;
     DBuf<float> rn2;
-    DBuf<uint32_t> slist;
-    DBuf<unsigned> scount;
     ScreenArgs sa{};
     if (screen) {
         MC_TRY(xb.alloc(a.n * a.d / 8, st));
         MC_TRY(rn2.alloc(a.n, st));
-        MC_TRY(slist.alloc(a.n, st));
-        MC_TRY(scount.alloc(1, st));
         MC_TRY(launch_to_bf16_flat8(a.X, a.n * a.d / 8, xb.p, sms, st));
         MC_TRY(launch_row_sums_dense(a.X, a.n, a.d, nullptr, rn2.p, st));
         const double g = double(a.d + 2) * 0x1p-24 / (1.0 - double(a.d + 2) * 0x1p-24);
@@ -1361,14 +1394,12 @@ static int run_kmeanspp_launches(const KmppArgs &a0, const double *u_dev, double
         sa.norm_up = std::nextafter(float(1.0 + double(a.d + 4) * 0x1p-24), 2.0f);
         sa.one_m_g = std::nextafter(float(1.0 - g), 0.0f);
         sa.one_p_2g = std::nextafter(float(1.0 + 2.0 * g), 2.0f);
-        sa.list = slist.p;
-        sa.count = scount.p;
     }
     DetInput in{a.w ? DET_F64_W : DET_F64, a.dist, nullptr, a.w, a.n};
     for (uint32_t ci = 1; ci < a.k; ++ci) {
-        MC_TRY(launch_det_draw(in, chunk_tmp, u_dev + ci, 0.0, 1, a.dist, a.newc, st));
+        MC_TRY(launch_det_draw_blocks(in, a.blk, chunk_tmp, ticket.p, u_dev + ci, a.dist, a.newc, st));
         if (screen) {
-            MC_TRY(screened_round(a, ci, sa, sms, st));
+            MC_TRY(screened_round(a, ci, sa, st));
             continue;
         }
         if (prune) {
@@ -1381,7 +1412,6 @@ static int run_kmeanspp_launches(const KmppArgs &a0, const double *u_dev, double
             k_kmpp_scatter<<<64, 256, 0, st>>>(a), note_launch();
         }
         MC_TRY(update(a, 0, ci, sms, st));
-        if (a.csr && !fused) k_kmpp_zero<<<1, 1, 0, st>>>(a), note_launch();
     }
     MC_CUDA_TRY(cudaGetLastError());
     return MC_OK;

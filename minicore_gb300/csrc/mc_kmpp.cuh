@@ -31,6 +31,9 @@ struct KmppArgs {
     // center to each earlier center, and the relative error bound of an FP32 row distance
     const double *cgap = nullptr;
     double prune_g = 0.0;
+    // optional: blk[b] = pairwise sum of (w *) dist over rows [32b, 32b + 32), kept current by
+    // every update (launch_det_draw_blocks draws from it)
+    double *blk = nullptr;
 };
 
 int run_kmeanspp(const KmppArgs &a, const double *u_dev, double *chunk_tmp, int sms, cudaStream_t st);
