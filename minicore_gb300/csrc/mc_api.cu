@@ -119,8 +119,11 @@ static int copy_out(T *dst, const T *src, size_t count, cudaStream_t st) {
 
 // CSR structure check (every kernel relies on it): indptr[0] == 0, nondecreasing,
 // indptr[n] == nnz, column indices < d and strictly increasing within each row.
-__global__ void k_validate_csr(const uint64_t *indptr, const uint32_t *idx, uint64_t n, uint64_t d, uint64_t nnz,
-                               int *bad) {
+// One thread per row: rows of a few entries (5 a row, 80,000 rows: 3.6 us against 30 us with a
+// warp per row).
+__global__ void __launch_bounds__(256) k_validate_csr_short(const uint64_t *__restrict__ indptr,
+                                                            const uint32_t *__restrict__ idx, uint64_t n, uint64_t d,
+                                                            uint64_t nnz, int *bad) {
     const uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
     if (i == 0 && (indptr[0] != 0 || indptr[n] != nnz)) atomicExch(bad, 1);
     if (i >= n) return;
@@ -137,12 +140,59 @@ __global__ void k_validate_csr(const uint64_t *indptr, const uint32_t *idx, uint
     }
 }
 
+// One warp per row, lanes over its entries: coalesced (1500 entries a row, 100,000 rows: 0.19 ms
+// against 0.83 ms with a thread per row, whose loads touch 32 rows each).
+__global__ void __launch_bounds__(256) k_validate_csr(const uint64_t *__restrict__ indptr,
+                                                      const uint32_t *__restrict__ idx, uint64_t n, uint64_t d,
+                                                      uint64_t nnz, int *bad) {
+    const int lane = threadIdx.x & 31;
+    const uint64_t nw = (gridDim.x * uint64_t(blockDim.x)) >> 5;
+    const uint64_t w0 = (blockIdx.x * uint64_t(blockDim.x) + threadIdx.x) >> 5;
+    if (w0 == 0 && lane == 0 && (indptr[0] != 0 || indptr[n] != nnz)) atomicExch(bad, 1);
+    // 32 rows' offsets at a time, one per lane
+    for (uint64_t g0 = w0 * 32; g0 < n; g0 += nw * 32) {
+        const uint64_t i = g0 + lane;
+        uint64_t bm = 0, em = 0;
+        if (i < n) {
+            bm = indptr[i];
+            em = indptr[i + 1];
+            if (em < bm || em > nnz) {
+                atomicExch(bad, 2);
+                em = bm = 0;
+            }
+        }
+        const int rows = int(umin64(32, n - g0));
+        for (int r = 0; r < rows; ++r) {
+            const uint64_t b = __shfl_sync(0xffffffffu, bm, r), e = __shfl_sync(0xffffffffu, em, r);
+            bool wrong = false;
+            long long before = -1;  // the entry before the 256 at hand
+            for (uint64_t p0 = b; p0 < e; p0 += 256) {
+                uint32_t j[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) j[u] = p0 + 32 * u + lane < e ? idx[p0 + 32 * u + lane] : 0xffffffffu;
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const uint32_t up = __shfl_up_sync(0xffffffffu, j[u], 1);
+                    const long long prev = lane ? (long long)up : before;
+                    if (p0 + 32 * u + lane < e) wrong |= j[u] >= d || (long long)j[u] <= prev;
+                    before = __shfl_sync(0xffffffffu, j[u], 31);
+                }
+            }
+            if (wrong) atomicExch(bad, 3);
+        }
+    }
+}
+
 static int validate_csr(const uint64_t *indptr, const uint32_t *idx, uint64_t n, uint64_t d, uint64_t nnz,
                         cudaStream_t st) {
     DBuf<int> flag;
     MC_TRY(flag.alloc(1, st));
     MC_CUDA_TRY(cudaMemsetAsync(flag.p, 0, sizeof(int), st));
-    k_validate_csr<<<unsigned((n + 255) / 256), 256, 0, st>>>(indptr, idx, n, d, nnz, flag.p), note_launch();
+    if (nnz < 16 * n)
+        k_validate_csr_short<<<unsigned((n + 255) / 256), 256, 0, st>>>(indptr, idx, n, d, nnz, flag.p), note_launch();
+    else
+        k_validate_csr<<<unsigned(umin64((n + 255) / 256, 152 * 8)), 256, 0, st>>>(indptr, idx, n, d, nnz, flag.p),
+            note_launch();
     MC_CUDA_TRY(cudaGetLastError());
     int bad = 0;
     MC_CUDA_TRY(cudaMemcpyAsync(&bad, flag.p, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -1280,7 +1330,7 @@ static int job_create_impl(mc_context *ctx, const mc_matrix *X, const float *cen
         // SQRL2 reads no row sums (the prior does not enter it)
         MC_TRY(launch_row_sums_dense(j->M.X, n, d, msr == SQRL2 ? nullptr : j->rowsum.p, j->rownorm.p, st));
     } else {
-        MC_TRY(launch_row_sums_csr(j->M.vals, j->M.indptr, n, j->rowsum.p, st));
+        MC_TRY(launch_row_sums_csr(j->M.vals, j->M.indptr, n, j->M.nnz, j->rowsum.p, st));
     }
     if (j->M.kind == MC_CSR_F32 && msr == JSD)
         MC_TRY(build_rinc_groups(j->rowsum.p, n, d, j->M.nnz, float(prior), st, j->grp, j->gval, j->ngrp));
@@ -1328,6 +1378,8 @@ static int job_create_impl(mc_context *ctx, const mc_matrix *X, const float *cen
         a.asn = j->asn.p;
         a.center_ids = ids.p;
         a.newc = newc.p;
+        KmppCsrWork cw;
+        MC_TRY(kmpp_csr_prepare(a, cw, j->M.nnz, ctx->sms, st));
         MC_TRY(run_kmeanspp(a, u.p, tmp.p, ctx->sms, st));
         MC_TRY(launch_gather_rows(j->M.kind == MC_CSR_F32, j->M.X, j->M.vals, j->M.idx, j->M.indptr, d, ids.p, k,
                                   j->C.p, st));
@@ -2224,7 +2276,7 @@ static int kmeanspp_impl(mc_context *ctx, const mc_matrix *X, uint32_t k, int ms
         MC_TRY(w.alloc(n, st));
         MC_CUDA_TRY(cudaMemcpyAsync(w.p, weights, n * sizeof(double), cudaMemcpyDefault, st));
     }
-    if (M.kind != MC_DENSE_F32) MC_TRY(launch_row_sums_csr(M.vals, M.indptr, n, rowsum.p, st));
+    if (M.kind != MC_DENSE_F32) MC_TRY(launch_row_sums_csr(M.vals, M.indptr, n, M.nnz, rowsum.p, st));
     else if (msr != SQRL2) MC_TRY(launch_row_sums_dense(M.X, n, d, rowsum.p, nullptr, st));  // SQRL2 reads none
     KmppArgs a;
     a.msr = msr;
@@ -2256,6 +2308,8 @@ static int kmeanspp_impl(mc_context *ctx, const mc_matrix *X, uint32_t k, int ms
     a.asn = asnb.p;
     a.center_ids = ids.p;
     a.newc = newc.p;
+    KmppCsrWork cw;
+    MC_TRY(kmpp_csr_prepare(a, cw, M.nnz, ctx->sms, st));
     if (local_trials > 1) MC_TRY(run_kmeanspp_greedy(a, local_trials, seed, tmp.p, ctx->sms, st));
     else MC_TRY(run_kmeanspp(a, u.p, tmp.p, ctx->sms, st));
     if (lspp_rounds) MC_TRY(run_lspp(ctx, X, a, k, msr, prior, lspp_rounds, seed, ids.p, asnb.p, dist.p, tmp.p, st));

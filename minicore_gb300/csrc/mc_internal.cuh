@@ -254,6 +254,7 @@ int launch_det_draw_blocks(const DetInput &in, const double *blk, double *chunk_
 
 // dense + CSR row statistics
 int launch_row_sums_dense(const float *X, uint64_t n, uint64_t d, double *rowsum, float *rownorm, cudaStream_t st);
-int launch_row_sums_csr(const float *vals, const uint64_t *indptr, uint64_t n, double *rowsum, cudaStream_t st);
+int launch_row_sums_csr(const float *vals, const uint64_t *indptr, uint64_t n, uint64_t nnz, double *rowsum,
+                        cudaStream_t st);
 
 }  // namespace mc

@@ -291,6 +291,22 @@ __global__ void __launch_bounds__(256) k_kmpp_csr(const KmppArgs a, int first, u
     }
 }
 
+// CSR rows against the new center in O(nnz) per row (SQRL2, L1, MKL, Hellinger; rows whose
+// pair keeps the prior pv = prior): per-center FP64 constants over all columns plus a float
+// sum over the row's nonzeros, the arithmetic of the sparse-dot assignment kernel:
+//   SQRL2  key = max(K0 + sum x (x - 2c), 0)                  K0 = sum c^2
+//   L1     key = (K0 + sum |c' - (x+pv)| - |c' - pv|) / 2     K0 = sum |c' - pv|, c' = c + pv
+//   MKL    key = K0 - log(rinc) K1 + sum a (log rinc - log b) K0 = sum a log a, K1 = sum a
+//   Hell.  key = sqrt(K0 - 2 s K1 + d s^2 + sum ((t - sqrt b)^2 - (t - s)^2))
+//          t = sqrt a (float), s = sqrt(rinc), K0 = sum t^2, K1 = sum t; the zero columns'
+//          part sum (t - s)^2 is formed whole and the nonzero terms in FP64, so a row equal
+//          to the center gets a distance near 0 (a sum of a + b - 2 sqrt(ab) cancels to the
+//          float rounding of its terms, which the square root lifts to ~1e-4)
+//   JSD    key = (Z[g] + sum (b log b - r log r) + sum (m0 log(m0/2) - m1 log(m1/2))) / 2
+//          m0 = a + r, m1 = a + b, r = rinc of the row's group g, Z[g] = sum over all
+//          columns of f(a, r) (k_kmpp_jsd_zcol)
+// with a = c * lhrsi + lhinc (center side), b = x * rhrsi + rhinc (row side).  Rows whose pair
+// moves the prior to the smallest-pv floor take the column loop of k_kmpp_csr.
 // Block sums of the per-thread FP64 partials (s0, s1) of a 1024-thread CTA: a pairwise tree
 // over the 32 lanes of each warp (shfl_xor), then over the 32 warp totals; warps that held no
 // column add nothing (their totals are 0).  Every thread gets the sums.  A dependent FP64 add
@@ -331,63 +347,416 @@ __device__ __forceinline__ void kp_block_sum2(double s0, double s1, uint64_t d, 
     u1 = w1[32];
 }
 
-// CSR rows against the new center in O(nnz) per row (SQRL2, L1, MKL, Hellinger; rows whose
-// pair keeps the prior pv = prior): per-center FP64 constants over all columns plus a float
-// sum over the row's nonzeros, the arithmetic of the sparse-dot assignment kernel:
-//   SQRL2  key = max(K0 + sum x (x - 2c), 0)                  K0 = sum c^2
-//   L1     key = (K0 + sum |c' - (x+pv)| - |c' - pv|) / 2     K0 = sum |c' - pv|, c' = c + pv
-//   MKL    key = K0 - log(rinc) K1 + sum a (log rinc - log b) K0 = sum a log a, K1 = sum a
-//   Hell.  key = sqrt(K0 - 2 s K1 + d s^2 + sum ((t - sqrt b)^2 - (t - s)^2))
-//          t = sqrt a (float), s = sqrt(rinc), K0 = sum t^2, K1 = sum t; the zero columns'
-//          part sum (t - s)^2 is formed whole and the nonzero terms in FP64, so a row equal
-//          to the center gets a distance near 0 (a sum of a + b - 2 sqrt(ab) cancels to the
-//          float rounding of its terms, which the square root lifts to ~1e-4)
-//   JSD    key = (Z[g] + sum (b log b - r log r) + sum (m0 log(m0/2) - m1 log(m1/2))) / 2
-//          m0 = a + r, m1 = a + b, r = rinc of the row's group g, Z[g] = sum over all
-//          columns of f(a, r) (k_kmpp_jsd_zcol)
-// with a = c * lhrsi + lhinc (center side), b = x * rhrsi + rhinc (row side).  Rows whose pair
-// moves the prior to the smallest-pv floor take the column loop of k_kmpp_csr.
-// k_kmpp_center_prep (one CTA) writes ct (c, c', a or sqrt a per column) and K0, K1: thread t
-// adds columns t, t+1024, ... in FP64; the 32 lanes of a warp, then the 32 warps, are added by
-// pairwise trees (kp_block_sum2).
+// ------------------------------------------------------------------------------------
+// CSR rounds.  A warp takes 32 rows at a time: lane l evaluates row g0 + l's skip test and
+// FP64 cost (a warp-wide FP64 instruction costs the SM's FP64 pipe the same whatever its
+// active lanes, so these run once per 32 rows), and the warp walks each row's entries together
+// (lanes strided over the entries, a butterfly for the float sum).  Rows go four at a time:
+// their first 32 entries are loaded together before any of them is used, so a short row does
+// not cost a memory round trip of its own.
+//
+// What depends on the row alone is taken from arrays written once per run (kmpp_csr_prepare):
+// rowc[i] = (float(rowsum + prior_sum), rsi, rinc, aux), and per entry the row side of its
+// term, rv[p] (MKL log b, Hellinger sqrt b, JSD b; b = x rsi + rinc), so that a round takes no
+// logarithm per entry for MKL: 100,000 x 20,000 rows of 1500 entries 350 -> 225 us per round
+// (1.2 GB: 177 us at the copy rate; the center side sits in shared memory).  They hold while the pair's pv is the prior itself
+// (checked per pair); other pairs take the full scalars and the column loop.
+// ------------------------------------------------------------------------------------
+
+// transform of a row entry's value x (b = x rsi + rinc, or x + pv for L1)
 template <int MSR>
-__global__ void __launch_bounds__(1024) k_kmpp_center_prep(const KmppArgs a) {
-    __shared__ double w0[33], w1[33];
+__device__ __forceinline__ float kp_row_value(float x, float fp, float rsi, float rinc) {
+    if (MSR == SQRL2) return x;
+    if (MSR == L1) return x + fp;
+    const float b = x * rsi + rinc;
+    if (MSR == MKL) return logf(b);
+    if (MSR == HELLINGER) return sqrtf(b);
+    return b;
+}
+
+template <int MSR>
+__global__ void __launch_bounds__(256) k_kmpp_csr_prepare(const KmppArgs a, float4 *rowc, float *rv, double *brow) {
+    const int lane = threadIdx.x & 31;
+    const uint64_t nw = (gridDim.x * uint64_t(blockDim.x)) >> 5;
+    const float fp = float(a.prior);
+    for (uint64_t i = (blockIdx.x * uint64_t(blockDim.x) + threadIdx.x) >> 5; i < a.n; i += nw) {
+        float rsi = 0.f, rinc = 0.f;
+        const double rs = a.rowsum[i];
+        side_scalars(fp, rs, a.d, rsi, rinc);
+        if (lane == 0) {
+            float aux = 0.f;
+            if (MSR == MKL) aux = logf(rinc);
+            else if (MSR == HELLINGER) aux = sqrtf(rinc);
+            else if (MSR == JSD) aux = rinc * logf(rinc);
+            rowc[i] = make_float4(float(rs + a.prior_sum), rsi, rinc, aux);
+        }
+        if (!rv && !brow) continue;  // whole warp
+        const float rlr = (MSR == JSD) ? rinc * logf(rinc) : 0.f;
+        double bsum = 0.0;
+        for (uint64_t p = a.indptr[i] + lane; p < a.indptr[i + 1]; p += 32) {
+            const float b = kp_row_value<MSR>(a.vals[p], fp, rsi, rinc);
+            if (rv) rv[p] = b;
+            if (MSR == JSD) bsum = bsum + double(b * logf(b) - rlr);
+        }
+        if (MSR == JSD && brow) {
+#pragma unroll
+            for (int m = 16; m >= 1; m >>= 1) bsum = bsum + __shfl_xor_sync(0xffffffffu, bsum, m);
+            if (lane == 0) brow[i] = bsum;
+        }
+    }
+}
+
+// one entry of the O(nnz) form (kp_nnz formulas below): cj = transformed center value
+template <int MSR>
+__device__ __forceinline__ void kp_nnz_term(float &acc, double &bsum, float cj, float x, float v, float fp, float rinc,
+                                            float aux) {
+    if (MSR == SQRL2) {
+        acc = fmaf(x, x - 2.f * cj, acc);
+    } else if (MSR == L1) {
+        acc = acc + (fabsf(cj - v) - fabsf(cj - fp));
+    } else if (MSR == MKL) {
+        acc = fmaf(cj, aux - v, acc);
+    } else if (MSR == JSD) {
+        const float m0 = cj + rinc, m1 = cj + v;
+        acc = acc + (m0 * logf(m0 * 0.5f) - m1 * logf(m1 * 0.5f));
+    } else {
+        // (sqrt a - sqrt b)^2 - (sqrt a - sqrt r)^2 in FP64 from the float roots
+        const double dd = double(cj) - double(v), de = double(cj) - double(aux);
+        bsum = bsum + (dd * dd - de * de);
+    }
+}
+
+// the column-loop form: kp_elem with the center side (p, q) and the row side (b, lb) given
+//   SQRL2 (c, -) (x, -)   L1 (c + pv, -) (x + pv, -)   Hellinger (sqrt a, -) (sqrt b, -)
+//   MKL (a, log a) (-, log b)   JSD (a, a log a) (b, b log b)
+template <int MSR>
+__device__ __forceinline__ float kp_elem_pre(float acc, float2 c, float b, float lb) {
+    if (MSR == SQRL2 || MSR == HELLINGER) {
+        const float df = c.x - b;
+        return fmaf(df, df, acc);
+    }
+    if (MSR == L1) return acc + fabsf(c.x - b);
+    if (MSR == MKL) return fmaf(c.x, c.y - lb, acc);
+    const float m = c.x + b;
+    const float t = (c.y + lb) - m * logf(m * 0.5f);
+    return acc + t;
+}
+
+// the rows of one round, RB at a time (8 in the column loop; 4 where a CTA of 1024 threads or
+// the loop over a long row's entries needs the registers: 8 there took 35 us instead of 20 at
+// 80,000 x 512, 5 entries a row).  COLS: the column-loop form (cp[j] = center side per column); else
+// the O(nnz) form (ct[j], constants K0, K1).  raw: the densified center row.
+template <int MSR, bool COLS, int RB>
+__device__ __forceinline__ void kp_csr_rows(const KmppArgs &a, int first, uint32_t round, uint64_t c, const float2 *cp,
+                                            const float *ct, const float *raw, double K0, double K1) {
+    const int lane = threadIdx.x & 31;
+    // 32-row groups go round the CTAs first: every SM has its share whatever n
+    const uint64_t warp = uint64_t(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    const uint64_t nwarps = (gridDim.x * uint64_t(blockDim.x)) >> 5;
+    const double csum = a.rowsum[c];
+    const float fp = float(a.prior);
+    const float lhsum0 = float(csum + a.prior_sum);
+    // entries are read as rv where that array exists (SQRL2: the values themselves)
+    const float *src = (MSR != SQRL2 && a.rv) ? a.rv : a.vals;
+    const bool pre = MSR == SQRL2 || a.rv != nullptr;
+    for (uint64_t g0 = warp * 32; g0 < a.n; g0 += nwarps * 32) {
+        const uint64_t my = g0 + uint64_t(lane);
+        const bool go = my < a.n && (first || (my != c && !(a.dist[my] <= 0.0)));
+        float4 rc = make_float4(0.f, 0.f, 0.f, 0.f);
+        uint64_t pbm = 0;
+        uint32_t lenm = 0;
+        bool fastm = true;
+        if (go) {
+            rc = a.rowc[my];
+            pbm = a.indptr[my];
+            lenm = uint32_t(a.indptr[my + 1] - pbm);
+            // pair_scalars keeps pv = prior unless it is below the smallest pv of the sums
+            fastm = MSR == SQRL2 || !(fp < 7.0069e-42f * (lhsum0 + rc.x));
+        }
+        float accm = 0.f;    // lane l: row g0 + l's float sum
+        double bsumm = 0.0;  // lane l: row g0 + l's FP64 sum (Hellinger)
+        const unsigned todo = __ballot_sync(0xffffffffu, go), fastb = __ballot_sync(0xffffffffu, fastm);
+        for (int r0 = 0; r0 < 32; r0 += RB) {
+            if (!((todo >> r0) & ((1u << RB) - 1u))) continue;
+            uint64_t pb[RB];
+            uint32_t len[RB], col[RB];
+            float x[RB], rsi[RB], rinc[RB], aux[RB], acc[RB];
+#pragma unroll
+            for (int u = 0; u < RB; ++u) {
+                pb[u] = __shfl_sync(0xffffffffu, pbm, r0 + u);
+                len[u] = __shfl_sync(0xffffffffu, lenm, r0 + u);
+                rsi[u] = __shfl_sync(0xffffffffu, rc.y, r0 + u);
+                rinc[u] = __shfl_sync(0xffffffffu, rc.z, r0 + u);
+                aux[u] = __shfl_sync(0xffffffffu, rc.w, r0 + u);
+                acc[u] = 0.f;
+                if (uint32_t(lane) < len[u]) {
+                    col[u] = __ldg(a.idx + pb[u] + lane);
+                    x[u] = __ldg(src + pb[u] + lane);
+                }
+            }
+            if (COLS) {
+                float b0[RB], lb0[RB];
+#pragma unroll
+                for (int u = 0; u < RB; ++u) {
+                    // the row side of a zero entry
+                    const float z = 0.f * rsi[u] + rinc[u];
+                    b0[u] = MSR == SQRL2 ? 0.f : MSR == L1 ? 0.f + fp : MSR == HELLINGER ? sqrtf(z) : z;
+                    lb0[u] = MSR == MKL ? logf(z) : MSR == JSD ? z * logf(z) : 0.f;
+                }
+                for (uint64_t j = lane; j < a.d; j += 32) {
+                    const float2 q = cp[j];
+#pragma unroll
+                    for (int u = 0; u < RB; ++u) acc[u] = kp_elem_pre<MSR>(acc[u], q, b0[u], lb0[u]);
+                }
+                // entries: acc + (term of the entry - term of a zero)
+                auto entry = [&](int u, uint32_t j, float xv) {
+                    const float v = pre ? xv : kp_row_value<MSR>(xv, fp, rsi[u], rinc[u]);
+                    const float2 q = cp[j];
+                    const float lb = MSR == MKL ? v : MSR == JSD ? v * logf(v) : 0.f;
+                    const float t1 = kp_elem_pre<MSR>(0.f, q, v, lb);
+                    const float t0 = kp_elem_pre<MSR>(0.f, q, b0[u], lb0[u]);
+                    acc[u] = acc[u] + (t1 - t0);
+                };
+#pragma unroll
+                for (int u = 0; u < RB; ++u) {
+                    if (uint32_t(lane) < len[u]) entry(u, col[u], x[u]);
+                    for (uint32_t p = uint32_t(lane) + 32; p < len[u]; p += 32)
+                        entry(u, a.idx[pb[u] + p], src[pb[u] + p]);
+                }
+            } else {
+#pragma unroll
+                for (int u = 0; u < RB; ++u) {
+                    double bsum = 0.0;
+                    auto entry = [&](uint32_t j, float xv) {
+                        const float v = pre ? xv : kp_row_value<MSR>(xv, fp, rsi[u], rinc[u]);
+                        kp_nnz_term<MSR>(acc[u], bsum, ct[j], xv, v, fp, rinc[u], aux[u]);
+                    };
+                    if (uint32_t(lane) < len[u]) entry(col[u], x[u]);
+                    // the rest of a long row, eight loads in flight
+                    uint32_t p = uint32_t(lane) + 32;
+                    for (; p + 7 * 32 < len[u]; p += 8 * 32) {
+                        uint32_t cj[8];
+                        float xj[8];
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) {
+                            cj[e] = __ldg(a.idx + pb[u] + p + 32 * e);
+                            xj[e] = __ldg(src + pb[u] + p + 32 * e);
+                        }
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) entry(cj[e], xj[e]);
+                    }
+                    for (; p < len[u]; p += 32) entry(a.idx[pb[u] + p], src[pb[u] + p]);
+                    if (MSR == HELLINGER) {
+#pragma unroll
+                        for (int m = 16; m >= 1; m >>= 1) bsum = bsum + __shfl_xor_sync(0xffffffffu, bsum, m);
+                        if (lane == r0 + u) bsumm = bsum;
+                    }
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < RB; ++u) {
+                if (!((fastb >> (r0 + u)) & 1u) && ((todo >> (r0 + u)) & 1u)) {
+                    // the pair's own pv: every column with the full scalars
+                    const PairScalars s = pair_scalars(a.prior, a.prior_sum, a.rowsum[g0 + r0 + u], csum, a.d);
+                    float t = 0.f;
+                    for (uint64_t j = lane; j < a.d; j += 32) kp_elem<MSR>(t, raw[j], 0.f, s);
+                    for (uint32_t p = lane; p < len[u]; p += 32) {
+                        const float cj = raw[a.idx[pb[u] + p]];
+                        float t1 = 0.f, t0 = 0.f;
+                        kp_elem<MSR>(t1, cj, a.vals[pb[u] + p], s);
+                        kp_elem<MSR>(t0, cj, 0.f, s);
+                        t = t + (t1 - t0);
+                    }
+                    acc[u] = t;
+                }
+#pragma unroll
+                for (int m = 16; m >= 1; m >>= 1) acc[u] = acc[u] + __shfl_xor_sync(0xffffffffu, acc[u], m);
+                if (lane == r0 + u) accm = acc[u];
+            }
+        }
+        double v = 0.0;
+        if (!go) {
+        } else if (!COLS && fastm) {
+            if (MSR == SQRL2) {
+                const double t = K0 + double(accm);
+                v = double(float(t < 0.0 ? 0.0 : t));
+            } else if (MSR == L1) {
+                v = double(float(K0 + double(accm)) * 0.5f) * 2.0;
+            } else if (MSR == MKL) {
+                v = double(post_divergence(float(K0 - double(rc.w) * K1 + double(accm))));
+            } else if (MSR == JSD) {
+                v = double(post_divergence(float((a.cconst[a.grp[my]] + a.brow[my] + double(accm)) * 0.5)));
+            } else {
+                const double sr = double(rc.w);
+                const double t = (K0 - 2.0 * sr * K1 + double(a.d) * sr * sr) + bsumm;
+                v = double(float(sqrt(t < 0.0 ? 0.0 : t))) * kSqrt1_2;
+            }
+        } else {
+            v = kp_cost<MSR>(accm);
+            if (MSR == SQRL2 && v < 0.0) v = 0.0;
+        }
+        kp_csr_row_out(a, first, round, c, my, go, v);
+    }
+}
+
+// the center's CSR row densified into shared memory (the whole CTA; a barrier before and after
+// the scatter), and the round's bookkeeping by CTA 0
+__device__ __forceinline__ void kp_densify(const KmppArgs &a, uint64_t c, uint32_t round, float *raw) {
+    for (uint64_t j = threadIdx.x; j < a.d; j += blockDim.x) raw[j] = 0.f;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        a.center_ids[round] = uint32_t(c);
+        a.asn[c] = round;
+    }
+    __syncthreads();
+    for (uint64_t p = a.indptr[c] + threadIdx.x; p < a.indptr[c + 1]; p += blockDim.x) raw[a.idx[p]] = a.vals[p];
+    __syncthreads();
+}
+
+// Column-loop rounds, one launch: every CTA forms the center side of all columns once (two
+// logarithms per (row, column) in the plain loop; 40,000 x 512, MKL: 60 -> 18 us per round).
+template <int MSR>
+__global__ void __launch_bounds__(256) k_kmpp_csr_cols(const KmppArgs a, int first, uint32_t round) {
+    extern __shared__ __align__(16) float sm_kp[];
+    float2 *cp = reinterpret_cast<float2 *>(sm_kp);
+    float *raw = sm_kp + 2 * a.d;
     const uint64_t c = *a.newc;
+    kp_densify(a, c, round, raw);
+    const float fp = float(a.prior);
+    float rsi = 0.f, inc = 0.f;
+    if (MSR != SQRL2 && MSR != L1) side_scalars(fp, a.rowsum[c], a.d, rsi, inc);
+    for (uint64_t j = threadIdx.x; j < a.d; j += blockDim.x) {
+        const float x = raw[j];
+        float2 q = make_float2(x, 0.f);
+        if (MSR == L1) {
+            q.x = x + fp;
+        } else if (MSR != SQRL2) {
+            const float av = x * rsi + inc;
+            q.x = MSR == HELLINGER ? sqrtf(av) : av;
+            q.y = MSR == MKL ? logf(av) : MSR == JSD ? av * logf(av) : 0.f;
+        }
+        cp[j] = q;
+    }
+    __syncthreads();
+    kp_csr_rows<MSR, true, 8>(a, first, round, c, cp, nullptr, raw, 0.0, 0.0);
+}
+
+// O(nnz) rounds with the center side in shared memory (SMEM) or global memory: two CTAs of 12
+// warps per SM leave a thread 85 registers, so eight entries of a row stay in flight
+constexpr int kNnzThreads = 384;
+
+template <int MSR, bool SMEM>
+__global__ void __launch_bounds__(kNnzThreads, 2) k_kmpp_csr_nnz(const KmppArgs a, int first, uint32_t round) {
+    extern __shared__ __align__(16) float sm_kp[];
+    const uint64_t c = *a.newc;
+    if (SMEM) {
+        for (uint64_t j = threadIdx.x; j < a.d; j += blockDim.x) sm_kp[j] = a.ct[j];
+        __syncthreads();
+    }
+    const double K0 = (MSR == JSD) ? 0.0 : a.cconst[0], K1 = (MSR == JSD) ? 0.0 : a.cconst[1];
+    kp_csr_rows<MSR, false, 4>(a, first, round, c, nullptr, SMEM ? sm_kp : a.ct, a.cbuf, K0, K1);
+}
+
+// center side of column value x and its FP64 terms
+template <int MSR>
+__device__ __forceinline__ float kp_center_value(float x, float pv, float rsi, float inc, double &s0, double &s1) {
+    if (MSR == SQRL2) {
+        s0 = s0 + double(x) * double(x);
+        return x;
+    }
+    if (MSR == L1) {
+        const float t = x + pv;
+        s0 = s0 + double(fabsf(t - pv));
+        return t;
+    }
+    const float av = x * rsi + inc;
+    if (MSR == JSD) return av;
+    if (MSR == MKL) {
+        s0 = s0 + double(av) * double(logf(av));
+        s1 = s1 + double(av);
+        return av;
+    }
+    const float t = sqrtf(av);
+    s0 = s0 + double(t) * double(t);
+    s1 = s1 + double(t);
+    return t;
+}
+
+// The center's row densified (cbuf), its transform (ct) and constants (cconst) by 32 CTAs: CTA
+// w takes the columns 32w + l + 1024 i, which are the terms of warp w of a 1024-thread block
+// (thread t adds columns t, t + 1024, ... in FP64), and the last CTA to finish adds the 32
+// warp totals by the same tree (kp_block_sum2), so the constants are those of one block; one
+// block's FP64 pipe took 34 us for 20,000 columns, after two launches that densified the row.
+// a.part: 64 doubles, a.ticket: a zero that is left zero.  self 0: k_kmpp_take and
+// k_kmpp_scatter have densified the row (more columns than fit shared memory).
+constexpr int kPrepCtas = 32;
+
+template <int MSR>
+__global__ void __launch_bounds__(128) k_kmpp_center_prep(const KmppArgs a, uint32_t round, int self) {
+    extern __shared__ __align__(16) float own[];  // [ceil(d / 1024)][32]
+    const uint64_t c = *a.newc;
+    const int t = threadIdx.x, lane = t & 31;
+    const uint32_t w = blockIdx.x;
+    const uint64_t per = (a.d + 1023) / 1024;
+    if (self) {
+        for (uint64_t e = t; e < per * 32; e += 128) own[e] = 0.f;
+        if (w == 0 && t == 0) {
+            a.center_ids[round] = uint32_t(c);
+            a.asn[c] = round;
+        }
+        __syncthreads();
+        for (uint64_t p = a.indptr[c] + t; p < a.indptr[c + 1]; p += 128) {
+            const uint32_t j = a.idx[p];
+            if (((j >> 5) & 31u) == w) own[uint64_t(j >> 10) * 32 + (j & 31u)] = a.vals[p];
+        }
+        __syncthreads();
+    }
+    auto value = [&](uint64_t e, uint64_t j) { return self ? own[e] : a.cbuf[j]; };
     const float pv = float(a.prior);
     float rsi = 0.f, inc = 0.f;
     if (MSR != SQRL2) side_scalars(pv, a.rowsum[c], a.d, rsi, inc);
-    double s0 = 0.0, s1 = 0.0;
-    for (uint64_t j = threadIdx.x; j < a.d; j += 1024) {
-        const float x = a.cbuf[j];
-        float t;
-        if (MSR == SQRL2) {
-            t = x;
-            s0 = s0 + double(x) * double(x);
-        } else if (MSR == L1) {
-            t = x + pv;
-            s0 = s0 + double(fabsf(t - pv));
-        } else {
-            const float av = x * rsi + inc;
-            if (MSR == JSD) {
-                t = av;
-            } else if (MSR == MKL) {
-                t = av;
-                s0 = s0 + double(av) * double(logf(av));
-                s1 = s1 + double(av);
-            } else {
-                t = sqrtf(av);
-                s0 = s0 + double(t) * double(t);
-                s1 = s1 + double(t);
+    if (t >= 32) {  // warps 1-3 write the row and its transform
+        for (uint64_t e = t - 32; e < per * 32; e += 96) {
+            const uint64_t j = (e >> 5) * 1024 + w * 32 + (e & 31);
+            if (j < a.d) {
+                double z0 = 0.0, z1 = 0.0;
+                const float x = value(e, j);
+                if (self) a.cbuf[j] = x;
+                a.ct[j] = kp_center_value<MSR>(x, pv, rsi, inc, z0, z1);
             }
         }
-        a.ct[j] = t;
+        return;
     }
-    double u0, u1;
-    kp_block_sum2(s0, s1, a.d, w0, w1, u0, u1);
-    if (threadIdx.x == 0 && MSR != JSD) {
-        a.cconst[0] = u0;
-        a.cconst[1] = u1;
+    if (MSR == JSD) return;  // no constants (k_kmpp_jsd_zcol)
+    double s0 = 0.0, s1 = 0.0;
+    for (uint64_t i = 0; i < per; ++i) {
+        const uint64_t j = i * 1024 + w * 32 + lane;
+        if (j < a.d) kp_center_value<MSR>(value(i * 32 + lane, j), pv, rsi, inc, s0, s1);
+    }
+#pragma unroll
+    for (int m = 16; m >= 1; m >>= 1) {
+        s0 = s0 + __shfl_xor_sync(0xffffffffu, s0, m);
+        s1 = s1 + __shfl_xor_sync(0xffffffffu, s1, m);
+    }
+    unsigned last = 0;
+    if (lane == 0) {
+        a.part[w] = s0;
+        a.part[32 + w] = s1;
+        __threadfence();
+        last = atomicAdd(a.ticket, 1u) == kPrepCtas - 1 ? 1u : 0u;
+    }
+    if (!__shfl_sync(0xffffffffu, last, 0)) return;
+    __threadfence();
+    s0 = __ldcg(a.part + lane);
+    s1 = __ldcg(a.part + 32 + lane);
+#pragma unroll
+    for (int m = 16; m >= 1; m >>= 1) {
+        s0 = s0 + __shfl_xor_sync(0xffffffffu, s0, m);
+        s1 = s1 + __shfl_xor_sync(0xffffffffu, s1, m);
+    }
+    if (lane == 0) {
+        a.cconst[0] = s0;
+        a.cconst[1] = s1;
+        *a.ticket = 0u;
     }
 }
 
@@ -411,192 +780,24 @@ __global__ void __launch_bounds__(256) k_kmpp_jsd_zcol(const KmppArgs a) {
     if (lane == 0) a.cconst[g] = t;
 }
 
-// the rows of one round: ct = transformed center, raw = densified center.  A warp takes 32
-// rows at a time: lane l evaluates row g0 + l's skip test, prior scalars and FP64 key (one
-// FP64 warp instruction per 32 rows), and the warp walks each row's nonzeros together (lanes
-// strided over the nonzeros, a butterfly for the float sum), as one warp per row did: the
-// arithmetic and its order are unchanged.
-template <int MSR>
-__device__ __forceinline__ void kp_nnz_rows(const KmppArgs &a, int first, uint32_t round, uint64_t c,
-                                            const float *ct, const float *raw, double K0, double K1) {
-    const int lane = threadIdx.x & 31;
-    const uint64_t warp = (blockIdx.x * uint64_t(blockDim.x) + threadIdx.x) >> 5;
-    const uint64_t nwarps = (gridDim.x * uint64_t(blockDim.x)) >> 5;
-    const double csum = a.rowsum[c];
-    const float fp = float(a.prior);
-    for (uint64_t g0 = warp * 32; g0 < a.n; g0 += nwarps * 32) {
-        const uint64_t my = g0 + uint64_t(lane);
-        const bool go = my < a.n && (first || (my != c && !(a.dist[my] <= 0.0)));
-        PairScalars sm = {0.f, 0.f, 0.f, 0.f, 0.f};
-        uint64_t pbm = 0, pem = 0;
-        float rincm = 0.f, rlm = 0.f, rlrm = 0.f, srincm = 0.f;
-        bool fastm = true;
-        if (go) {
-            sm = pair_scalars(a.prior, a.prior_sum, a.rowsum[my], csum, a.d);
-            pbm = a.indptr[my];
-            pem = a.indptr[my + 1];
-            fastm = MSR == SQRL2 || sm.pv == fp;
-            rincm = (MSR == JSD) ? a.gval[a.grp[my]] : sm.rhinc;
-            rlrm = (MSR == JSD) ? rincm * logf(rincm) : 0.f;
-            rlm = (MSR == MKL) ? logf(rincm) : 0.f;
-            srincm = (MSR == HELLINGER) ? sqrtf(rincm) : 0.f;
-        }
-        float accm = 0.f;     // lane l: row g0 + l's float sum
-        double bsumm = 0.0;   // lane l: row g0 + l's FP64 sum (Hellinger, JSD)
-        unsigned todo = __ballot_sync(0xffffffffu, go);
-        while (todo) {
-            const int r = __ffs(todo) - 1;
-            todo &= todo - 1;
-            const uint64_t pb = __shfl_sync(0xffffffffu, pbm, r), pe = __shfl_sync(0xffffffffu, pem, r);
-            const bool fast = __shfl_sync(0xffffffffu, fastm ? 1 : 0, r) != 0;
-            if (fast) {
-                const float rsi = __shfl_sync(0xffffffffu, sm.rhrsi, r);
-                const float rinc = __shfl_sync(0xffffffffu, rincm, r);
-                const float rlr = __shfl_sync(0xffffffffu, rlrm, r);
-                const float rl = __shfl_sync(0xffffffffu, rlm, r);
-                const float srinc = __shfl_sync(0xffffffffu, srincm, r);
-                float acc = 0.f;
-                double bsum = 0.0;
-#pragma unroll 4
-                for (uint64_t p = pb + lane; p < pe; p += 32) {
-                    const float x = a.vals[p];
-                    const float cj = ct[a.idx[p]];
-                    if (MSR == SQRL2) {
-                        acc = fmaf(x, x - 2.f * cj, acc);
-                    } else if (MSR == L1) {
-                        acc = acc + (fabsf(cj - (x + fp)) - fabsf(cj - fp));
-                    } else if (MSR == MKL) {
-                        acc = fmaf(cj, rl - logf(x * rsi + rinc), acc);
-                    } else if (MSR == JSD) {
-                        const float b = x * rsi + rinc;
-                        const float m0 = cj + rinc, m1 = cj + b;
-                        acc = acc + (m0 * logf(m0 * 0.5f) - m1 * logf(m1 * 0.5f));
-                        bsum = bsum + double(b * logf(b) - rlr);
-                    } else {
-                        // (sqrt a - sqrt b)^2 - (sqrt a - sqrt r)^2 in FP64 from the float roots
-                        const float b = x * rsi + rinc;
-                        const double dd = double(cj) - double(sqrtf(b)), de = double(cj) - double(srinc);
-                        bsum = bsum + (dd * dd - de * de);
-                    }
-                }
-#pragma unroll
-                for (int m = 16; m >= 1; m >>= 1) {
-                    acc = acc + __shfl_xor_sync(0xffffffffu, acc, m);
-                    if (MSR == HELLINGER || MSR == JSD) bsum = bsum + __shfl_xor_sync(0xffffffffu, bsum, m);
-                }
-                if (lane == r) {
-                    accm = acc;
-                    bsumm = bsum;
-                }
-            } else {
-                PairScalars s;
-                s.pv = __shfl_sync(0xffffffffu, sm.pv, r);
-                s.lhrsi = __shfl_sync(0xffffffffu, sm.lhrsi, r);
-                s.rhrsi = __shfl_sync(0xffffffffu, sm.rhrsi, r);
-                s.lhinc = __shfl_sync(0xffffffffu, sm.lhinc, r);
-                s.rhinc = __shfl_sync(0xffffffffu, sm.rhinc, r);
-                float acc = 0.f;
-                for (uint64_t j = lane; j < a.d; j += 32) kp_elem<MSR>(acc, raw[j], 0.f, s);
-                for (uint64_t p = pb + lane; p < pe; p += 32) {
-                    const float cj = raw[a.idx[p]];
-                    float t1 = 0.f, t0 = 0.f;
-                    kp_elem<MSR>(t1, cj, a.vals[p], s);
-                    kp_elem<MSR>(t0, cj, 0.f, s);
-                    acc = acc + (t1 - t0);
-                }
-#pragma unroll
-                for (int m = 16; m >= 1; m >>= 1) acc = acc + __shfl_xor_sync(0xffffffffu, acc, m);
-                if (lane == r) accm = acc;
-            }
-        }
-        double v = 0.0;
-        if (!go) {
-        } else if (fastm) {
-            float key;
-            if (MSR == SQRL2) {
-                double t = K0 + double(accm);
-                key = float(t < 0.0 ? 0.0 : t);
-                v = double(key);
-            } else if (MSR == L1) {
-                key = float(K0 + double(accm)) * 0.5f;
-                v = double(key) * 2.0;
-            } else if (MSR == MKL) {
-                key = post_divergence(float(K0 - double(rlm) * K1 + double(accm)));
-                v = double(key);
-            } else if (MSR == JSD) {
-                key = post_divergence(float((a.cconst[a.grp[my]] + bsumm + double(accm)) * 0.5));
-                v = double(key);
-            } else {
-                const double sr = double(srincm);
-                double t = (K0 - 2.0 * sr * K1 + double(a.d) * sr * sr) + bsumm;
-                key = float(sqrt(t < 0.0 ? 0.0 : t));
-                v = double(key) * kSqrt1_2;
-            }
-        } else {
-            v = kp_cost<MSR>(accm);
-            if (MSR == SQRL2 && v < 0.0) v = 0.0;
-        }
-        kp_csr_row_out(a, first, round, c, my, go, v);
-    }
-}
-
-template <int MSR>
-__global__ void __launch_bounds__(256) k_kmpp_csr_nnz(const KmppArgs a, int first, uint32_t round) {
-    const uint64_t c = *a.newc;
-    const double K0 = (MSR == JSD) ? 0.0 : a.cconst[0], K1 = (MSR == JSD) ? 0.0 : a.cconst[1];
-    kp_nnz_rows<MSR>(a, first, round, c, a.ct, a.cbuf, K0, K1);
-}
-
 // Small d (2 d floats of shared memory): one launch per round.  Every CTA densifies the new
-// center's CSR row into shared memory, forms ct and K0, K1 with the code and summation order
-// of k_kmpp_center_prep (1024 threads), then runs its share of the rows; CTA 0 also records
-// the center and zeroes its distance (k_kmpp_take / k_kmpp_zero).  Same results as the
-// three-launch sequence.
+// center's CSR row into shared memory, forms ct and K0, K1 with the summation order of
+// k_kmpp_center_prep, then runs its share of the rows.
 template <int MSR>
 __global__ void __launch_bounds__(1024) k_kmpp_csr_fused(const KmppArgs a, int first, uint32_t round) {
-    extern __shared__ float sm_kp[];
+    extern __shared__ __align__(16) float sm_kp[];
     float *raw = sm_kp, *ct = sm_kp + a.d;
     __shared__ double w0[33], w1[33];
     const uint64_t c = *a.newc;
-    const int tid = threadIdx.x;
-    for (uint64_t j = tid; j < a.d; j += 1024) raw[j] = 0.f;
-    __syncthreads();
-    for (uint64_t p = a.indptr[c] + tid; p < a.indptr[c + 1]; p += 1024) raw[a.idx[p]] = a.vals[p];
-    if (blockIdx.x == 0 && tid == 0) {
-        a.center_ids[round] = uint32_t(c);
-        a.asn[c] = round;
-    }
-    __syncthreads();
+    kp_densify(a, c, round, raw);
     const float pv = float(a.prior);
     float rsi = 0.f, inc = 0.f;
     if (MSR != SQRL2) side_scalars(pv, a.rowsum[c], a.d, rsi, inc);
     double s0 = 0.0, s1 = 0.0;
-    for (uint64_t j = tid; j < a.d; j += 1024) {
-        const float x = raw[j];
-        float t;
-        if (MSR == SQRL2) {
-            t = x;
-            s0 = s0 + double(x) * double(x);
-        } else if (MSR == L1) {
-            t = x + pv;
-            s0 = s0 + double(fabsf(t - pv));
-        } else {
-            const float av = x * rsi + inc;
-            if (MSR == MKL) {
-                t = av;
-                s0 = s0 + double(av) * double(logf(av));
-                s1 = s1 + double(av);
-            } else {
-                t = sqrtf(av);
-                s0 = s0 + double(t) * double(t);
-                s1 = s1 + double(t);
-            }
-        }
-        ct[j] = t;
-    }
+    for (uint64_t j = threadIdx.x; j < a.d; j += 1024) ct[j] = kp_center_value<MSR>(raw[j], pv, rsi, inc, s0, s1);
     double u0, u1;
     kp_block_sum2(s0, s1, a.d, w0, w1, u0, u1);
-    kp_nnz_rows<MSR>(a, first, round, c, ct, raw, u0, u1);
+    kp_csr_rows<MSR, false, 4>(a, first, round, c, nullptr, ct, raw, u0, u1);
 }
 
 __device__ __forceinline__ void kp_cp_async16(void *dst, const void *src, int src_bytes) {
@@ -814,8 +1015,50 @@ __global__ void __launch_bounds__(128) k_kmpp_dense_persist(const KmppArgs a, in
     }
 }
 
-// CSR update in one launch per round: the center row and its transform fit in 32 KB
+// CSR rounds: k_kmpp_csr_cols (no ct: the column loop), k_kmpp_csr_fused (ct and d <= 4096) or
+// k_kmpp_center_prep + k_kmpp_csr_nnz; each takes the center's row itself while it fits shared
+// memory.  Otherwise k_kmpp_take and k_kmpp_scatter densify it first, and the column loop is
+// k_kmpp_csr.
+constexpr uint64_t kKpColsMax = 16384;         // 3 d floats: 192 KB
+constexpr uint64_t kKpPrepMax = 1024ull * 1536;  // d / 32 floats: 192 KB
+constexpr uint64_t kKpCtMax = 49152;           // d floats: 192 KB
+
+template <int MSR>
+static int kmpp_csr_prepare_t(const KmppArgs &a, float4 *rowc, float *rv, double *brow, int sms, cudaStream_t st) {
+    k_kmpp_csr_prepare<MSR><<<unsigned(umin64((a.n + 7) / 8, uint64_t(sms) * 16)), 256, 0, st>>>(a, rowc, rv, brow),
+        note_launch();
+    MC_CUDA_TRY(cudaGetLastError());
+    return MC_OK;
+}
+
+int kmpp_csr_prepare(KmppArgs &a, KmppCsrWork &w, uint64_t nnz, int sms, cudaStream_t st) {
+    if (!a.csr) return MC_OK;
+    MC_TRY(w.rowc.alloc(a.n, st));
+    MC_TRY(w.part.alloc(64, st));
+    MC_TRY(w.ticket.alloc(1, st));
+    MC_CUDA_TRY(cudaMemsetAsync(w.ticket.p, 0, sizeof(unsigned), st));
+    if (a.msr == JSD) MC_TRY(w.brow.alloc(a.n, st));
+    // the entries' row side pays from a few rounds on; without the memory for it the rounds
+    // form it from the values each time
+    const bool uses = a.msr == MKL || a.msr == HELLINGER || a.msr == JSD;
+    if (uses && a.k >= 4 && nnz && w.rv.alloc(nnz, st) != MC_OK) cudaGetLastError();
+    a.rowc = w.rowc.p;
+    a.rv = w.rv.p;
+    a.brow = w.brow.p;
+    a.part = w.part.p;
+    a.ticket = w.ticket.p;
+    switch (a.msr) {
+        case SQRL2: return kmpp_csr_prepare_t<SQRL2>(a, w.rowc.p, w.rv.p, w.brow.p, sms, st);
+        case L1: return kmpp_csr_prepare_t<L1>(a, w.rowc.p, w.rv.p, w.brow.p, sms, st);
+        case HELLINGER: return kmpp_csr_prepare_t<HELLINGER>(a, w.rowc.p, w.rv.p, w.brow.p, sms, st);
+        case MKL: return kmpp_csr_prepare_t<MKL>(a, w.rowc.p, w.rv.p, w.brow.p, sms, st);
+        case JSD: return kmpp_csr_prepare_t<JSD>(a, w.rowc.p, w.rv.p, w.brow.p, sms, st);
+        default: return fail(MC_EUNSUPPORTED, "measure not supported");
+    }
+}
+
 static bool kmpp_csr_fused_ok(const KmppArgs &a) { return a.csr && a.msr != JSD && a.ct && a.d <= 4096; }
+static bool kmpp_self_take(const KmppArgs &a) { return a.csr && a.d <= (a.ct ? kKpPrepMax : kKpColsMax); }
 
 template <int MSR>
 static int update_t(const KmppArgs &a, int first, uint32_t round, int sms, cudaStream_t st) {
@@ -842,16 +1085,36 @@ static int update_t(const KmppArgs &a, int first, uint32_t round, int sms, cudaS
         }
         k_kmpp_dense<MSR, false><<<unsigned((a.n + 255) / 256), 256, 0, st>>>(b, first), note_launch();
     } else {
-        const unsigned blocks = unsigned(umin64((a.n + 7) / 8, uint64_t(sms) * 16));
-        if (MSR != JSD && a.ct && kmpp_csr_fused_ok(a)) {
-            const unsigned fb = unsigned(umin64((a.n + 31) / 32, uint64_t(sms) * 2));
-            k_kmpp_csr_fused<MSR><<<fb, 1024, 2 * a.d * sizeof(float), st>>>(a, first, round), note_launch();
+        const uint64_t groups = (a.n + 31) / 32;  // a warp each
+        if (kmpp_csr_fused_ok(a)) {
+            if constexpr (MSR != JSD) {
+                // every CTA forms the constants itself (FP64): one per SM while that is enough warps
+                const unsigned fb = unsigned(umin64(groups, uint64_t(sms) * (groups > uint64_t(sms) * 32 ? 2 : 1)));
+                k_kmpp_csr_fused<MSR><<<fb, 1024, 2 * a.d * sizeof(float), st>>>(a, first, round), note_launch();
+            }
         } else if (a.ct) {
-            k_kmpp_center_prep<MSR><<<1, 1024, 0, st>>>(a), note_launch();
+            const bool self = kmpp_self_take(a);
+            const size_t psm = self ? (a.d + 1023) / 1024 * 128 : 0;
+            MC_CUDA_TRY(cudaFuncSetAttribute(k_kmpp_center_prep<MSR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             int(kKpPrepMax / 1024 * 128)));
+            k_kmpp_center_prep<MSR><<<kPrepCtas, 128, psm, st>>>(a, round, self ? 1 : 0), note_launch();
             if (MSR == JSD) k_kmpp_jsd_zcol<<<unsigned((a.ngrp + 7) / 8), 256, 0, st>>>(a), note_launch();
-            k_kmpp_csr_nnz<MSR><<<blocks, 256, 0, st>>>(a, first, round), note_launch();
+            const unsigned blocks = unsigned(umin64(groups, uint64_t(sms) * 2));
+            if (a.d <= kKpCtMax) {
+                MC_CUDA_TRY(cudaFuncSetAttribute(k_kmpp_csr_nnz<MSR, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 int(kKpCtMax * sizeof(float))));
+                k_kmpp_csr_nnz<MSR, true><<<blocks, kNnzThreads, a.d * sizeof(float), st>>>(a, first, round), note_launch();
+            } else {
+                k_kmpp_csr_nnz<MSR, false><<<blocks, kNnzThreads, 0, st>>>(a, first, round), note_launch();
+            }
+        } else if (a.d <= kKpColsMax) {
+            MC_CUDA_TRY(cudaFuncSetAttribute(k_kmpp_csr_cols<MSR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             int(kKpColsMax * 12)));
+            k_kmpp_csr_cols<MSR><<<unsigned(umin64((groups + 7) / 8, uint64_t(sms) * 8)), 256, 3 * a.d * sizeof(float),
+                                   st>>>(a, first, round), note_launch();
         } else {
-            k_kmpp_csr<MSR><<<blocks, 256, 0, st>>>(a, first, round), note_launch();
+            k_kmpp_csr<MSR><<<unsigned(umin64((a.n + 7) / 8, uint64_t(sms) * 16)), 256, 0, st>>>(a, first, round),
+                note_launch();
         }
     }
     MC_CUDA_TRY(cudaGetLastError());
@@ -1364,8 +1627,8 @@ static int run_kmeanspp_launches(const KmppArgs &a0, const double *u_dev, double
     const unsigned tb = 256, tg = unsigned(umin64((a.d + tb - 1) / tb, 1024));
     MC_CUDA_TRY(cudaMemsetAsync(a.asn, 0, a.n * sizeof(uint32_t), st));
     k_kmpp_first<<<1, 1, 0, st>>>(u_dev, a.n, a.newc, a.center_ids), note_launch();
-    const bool fused = kmpp_csr_fused_ok(a);  // the update kernel takes the center itself
-    if (a.csr && !fused) {
+    const bool self = kmpp_self_take(a);  // the update takes the center's row itself
+    if (a.csr && !self) {
         k_kmpp_take<<<tg, tb, 0, st>>>(a, 0), note_launch();
         k_kmpp_scatter<<<64, 256, 0, st>>>(a), note_launch();
     }
@@ -1406,7 +1669,7 @@ static int run_kmeanspp_launches(const KmppArgs &a0, const double *u_dev, double
             k_kmpp_center_gap<<<unsigned((ci + 7) / 8), 256, 0, st>>>(a, ci, gap.p), note_launch();
             a.cgap = gap.p;
         }
-        if (a.csr && !fused) {
+        if (a.csr && !self) {
             // CSR centers are densified into cbuf; the dense update reads the center row itself
             k_kmpp_take<<<tg, tb, 0, st>>>(a, ci), note_launch();
             k_kmpp_scatter<<<64, 256, 0, st>>>(a), note_launch();
@@ -1460,8 +1723,8 @@ __global__ void k_kmpp_pick(const double *u, uint64_t n, uint64_t *out) {
 // distances to the first center)
 static int kmpp_add_candidate(const KmppArgs &b, int first, uint32_t round, int sms, cudaStream_t st) {
     const unsigned tb = 256, tg = unsigned(umin64((b.d + tb - 1) / tb, 1024));
-    const bool fused = kmpp_csr_fused_ok(b);
-    if (b.csr && !fused) {
+    const bool self = kmpp_self_take(b);
+    if (b.csr && !self) {
         k_kmpp_take<<<tg, tb, 0, st>>>(b, round), note_launch();
         k_kmpp_scatter<<<64, 256, 0, st>>>(b), note_launch();
     }

@@ -34,7 +34,23 @@ struct KmppArgs {
     // optional: blk[b] = pairwise sum of (w *) dist over rows [32b, 32b + 32), kept current by
     // every update (launch_det_draw_blocks draws from it)
     double *blk = nullptr;
+    // CSR rows: what depends on a row alone (kmpp_csr_prepare)
+    const float4 *rowc = nullptr;  // [n] float(rowsum + prior_sum), rsi, rinc, aux
+    const float *rv = nullptr;     // [nnz] row side of each entry's term, or null (formed from the value)
+    const double *brow = nullptr;  // [n] JSD: FP64 sum over the row's entries
+    double *part = nullptr;        // [64] center prep partials
+    unsigned *ticket = nullptr;    // zero between launches
 };
+
+struct KmppCsrWork {
+    DBuf<float4> rowc;
+    DBuf<float> rv;
+    DBuf<double> brow, part;
+    DBuf<unsigned> ticket;
+};
+// the arrays above, for CSR rows (before any round); no-op for dense rows
+int kmpp_csr_prepare(KmppArgs &a, KmppCsrWork &w, uint64_t nnz, int sms, cudaStream_t st);
+
 
 int run_kmeanspp(const KmppArgs &a, const double *u_dev, double *chunk_tmp, int sms, cudaStream_t st);
 // distances of every row to row *cand (see mc_kmpp.cu)
