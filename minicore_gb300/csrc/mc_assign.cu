@@ -17,6 +17,7 @@
 // center-side and row-side transforms are precomputed; otherwise (prior 0) every pair
 // recomputes them ("pair mode").
 #include "mc_assign.cuh"
+#include "mc_assign_dev.cuh"
 #include "mc_tune.cuh"
 
 namespace mc {
@@ -144,57 +145,6 @@ __global__ void k_row_scalars(const double *__restrict__ rowsum, uint64_t n, uin
 }
 
 // ------------------------------------------------------------------------------------
-// argmin bookkeeping: lexicographic (value, index); NaN at center 0 wins (the reference's
-// sequential scan then never moves off center 0), NaN elsewhere never wins.
-// ------------------------------------------------------------------------------------
-struct Best {
-    float v;
-    uint32_t j;
-};
-
-__device__ inline void best_init(Best &b) {
-    b.v = __int_as_float(0x7f800000);
-    b.j = 0xffffffffu;
-}
-
-__device__ inline void best_offer(Best &b, float v, uint32_t j) {
-    if (v != v) {
-        if (j != 0) return;
-        v = __int_as_float(0xff800000);  // -inf marks "NaN at center 0"
-    }
-    if (v < b.v || (v == b.v && j < b.j)) {
-        b.v = v;
-        b.j = j;
-    }
-}
-
-__device__ inline void best_merge_shfl(Best &b, int lanemask_xor) {
-    const float ov = __shfl_xor_sync(0xffffffffu, b.v, lanemask_xor);
-    const uint32_t oj = __shfl_xor_sync(0xffffffffu, b.j, lanemask_xor);
-    if (ov < b.v || (ov == b.v && oj < b.j)) {
-        b.v = ov;
-        b.j = oj;
-    }
-}
-
-// final value of a pair: compare key (float) and cost (double) per measure
-template <int MSR>
-__device__ inline float finish_key(float acc) {
-    if (MSR == SQRL2) return acc;
-    if (MSR == L1) return acc * 0.5f;
-    if (MSR == HELLINGER) return sqrtf(acc);
-    if (MSR == MKL) return post_divergence(acc);
-    return post_divergence(acc * 0.5f);  // JSD
-}
-
-template <int MSR>
-__device__ inline double key_to_cost(float key) {
-    if (MSR == L1) return double(key) * 2.0;
-    if (MSR == HELLINGER) return double(key) * kSqrt1_2;
-    return double(key);
-}
-
-// ------------------------------------------------------------------------------------
 // tiled kernel
 // ------------------------------------------------------------------------------------
 constexpr int kBK = 16;
@@ -242,19 +192,6 @@ __device__ inline void elem(float &acc, float c0, float c1, float x0, float x1, 
             const float t = (a * logf(a) + b * logf(b)) - m * logf(m * 0.5f);
             acc = acc + t;
         }
-    }
-}
-
-// row-side transform of a raw value x for the constant-prior path
-template <int MSR>
-__device__ inline void row_xform(float x, float pv, float rsi, float rinc, float &x0, float &x1) {
-    if (MSR == SQRL2) { x0 = x; x1 = 0.f; }
-    else if (MSR == L1) { x0 = x + pv; x1 = 0.f; }
-    else if (MSR == HELLINGER) { x0 = sqrtf(x * rsi + rinc); x1 = 0.f; }
-    else {
-        const float b = x * rsi + rinc;
-        if (MSR == MKL) { x0 = logf(b); x1 = 0.f; }
-        else { x0 = b; x1 = b * logf(b); }
     }
 }
 
@@ -1287,12 +1224,16 @@ static int tiled_t(const AssignArgs &a, bool pair, bool big, cudaStream_t st, bo
         constexpr int BM = 32;
         k_assign_tiled<MSR, true, 2, 2, CSR><<<unsigned((a.n + BM - 1) / BM), 256, 0, st>>>(a), note_launch();
     } else if (big) {
-        // SQRL2 with kp % 128 == 0: 8x8 register tiles (128 rows per CTA) or 4x4 (64 rows);
-        // same per-pair arithmetic, so the autotuner may pick either
+        // SQRL2 with kp % 128 == 0: 8x8 register tiles (128 rows per CTA) or 4x4 (64 rows), dense
+        // rows k_assign_dense or 8x8; same per-pair arithmetic, so the autotuner may pick either
         const std::string key = std::string("dense_sqrl2|") + (CSR ? "csr" : "dense") + "|k" +
                                 std::to_string(a.kp) + "|d" + tune_bucket(a.d) + "|n" + tune_bucket(a.n);
         return tune_launch(key, 2, 0, st, tune, [&](int v) -> int {
-            if (v == 0)
+            if (!CSR && v == 0) {
+                bool done = false;
+                return launch_assign_dense(a, st, &done);
+            }
+            if (v == (CSR ? 0 : 1))
                 k_assign_tiled<MSR, false, 8, 8, CSR><<<unsigned((a.n + 127) / 128), 256, 0, st>>>(a), note_launch();
             else
                 k_assign_tiled<MSR, false, 4, 4, CSR><<<unsigned((a.n + 63) / 64), 256, 0, st>>>(a), note_launch();
@@ -1316,6 +1257,11 @@ int launch_assign_tiled(const AssignArgs &a, bool csr, bool pair, cudaStream_t s
     if (a.n == 0) return MC_OK;
     // 8x8 register tiles for SQRL2 with many centers, 4x4 otherwise
     const bool big = (a.msr == SQRL2 && a.kp % 128 == 0);
+    if (!csr && !pair && !big) {
+        bool done = false;
+        MC_TRY(launch_assign_dense(a, st, &done));
+        if (done) return MC_OK;
+    }
     switch (a.msr) {
         case SQRL2:
             return csr ? tiled_t<SQRL2, true>(a, pair, big, st, tune) : tiled_t<SQRL2, false>(a, pair, big, st, tune);

@@ -53,6 +53,8 @@ int launch_row_scalars(const double *rowsum, uint64_t n, uint64_t d, float pv, f
 // tune: the autotuner may time kernel variants on the first call for a shape (callers that
 // must not synchronise or allocate pass false)
 int launch_assign_tiled(const AssignArgs &a, bool csr, bool pair, cudaStream_t st, bool tune = true);
+// dense rows, constant prior (mc_assign_dense.cu); *done = false: not covered there
+int launch_assign_dense(const AssignArgs &a, cudaStream_t st, bool *done);
 int launch_assign_sparse(const AssignArgs &a, cudaStream_t st, int sms, bool tune = true);
 // L1 over CSR rows in pair mode (prior 0): a walk over the union of nonzero columns,
 // bit-identical to the tiled kernel; work: l1_union_work_entries(k, d) floats
