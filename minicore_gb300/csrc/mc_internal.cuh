@@ -129,8 +129,14 @@ __host__ __device__ inline uint64_t det_leaves(uint64_t n) {
     while (p < det_chunks(n)) p <<= 1;
     return p;
 }
+constexpr uint64_t kDetWarp = 1024;        // elements per leaf of a sum over few elements
+constexpr uint64_t kDetSmemLeaves = 2048;  // tree in shared memory up to this many leaves
 // doubles of scratch that launch_det_sum / launch_det_draw need (the tree, heap layout)
-__host__ __device__ inline uint64_t det_tmp_size(uint64_t n) { return 2 * det_leaves(n); }
+__host__ __device__ inline uint64_t det_tmp_size(uint64_t n) {
+    const uint64_t chunks = 2 * det_leaves(n);
+    if (n > kDetWarp * kDetSmemLeaves) return chunks;
+    return 8 * chunks < 2 * kDetSmemLeaves ? 8 * chunks : 2 * kDetSmemLeaves;
+}
 
 // pairwise sum of 32 consecutive elements held one per lane; the result is in lane 0
 __device__ __forceinline__ double lane_pairwise32(double v) {

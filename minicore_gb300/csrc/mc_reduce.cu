@@ -62,8 +62,6 @@ __device__ void det_heap_build(double *T, uint64_t P, uint64_t G) {
     }
 }
 
-constexpr uint64_t kDetSmemLeaves = 2048;  // tree in shared memory up to this many leaves
-
 __global__ void __launch_bounds__(kDetThreads) k_det_final(double *tree, uint64_t P, uint64_t G, double *out) {
     __shared__ double sT[2 * kDetSmemLeaves];
     double *T = tree;
@@ -75,7 +73,43 @@ __global__ void __launch_bounds__(kDetThreads) k_det_final(double *tree, uint64_
     if (threadIdx.x == 0) *out = T[1];
 }
 
+// Totals of 1024 consecutive elements, one warp each: loaded coalesced, turned through shared
+// memory so that each lane adds its 32 consecutive elements (31 adds per 32 elements, as
+// k_det_chunks), then a pairwise tree over the lanes.  The leaves of the same tree three levels
+// lower: at 10,000 elements ten SMs share what k_det_chunks gives to two (8.4 -> 3.3 us).
+__global__ void __launch_bounds__(64) k_det_warps(DetInput in, double *leaves, uint64_t G) {
+    __shared__ double v[2][32 * 33];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint64_t g = uint64_t(blockIdx.x) * 2 + w;
+    if (g >= G) return;  // whole warp; no block barrier
+    const uint64_t b = g * kDetWarp;
+#pragma unroll
+    for (int r = 0; r < 32; ++r) {
+        const uint64_t i = b + uint64_t(r) * 32 + lane;
+        v[w][r * 33 + lane] = i < in.n ? in.get(i) : 0.0;
+    }
+    __syncwarp();
+    double e[32];
+#pragma unroll
+    for (int q = 0; q < 32; ++q) e[q] = v[w][lane * 33 + q];
+#pragma unroll
+    for (int sft = 1; sft < 32; sft <<= 1)
+#pragma unroll
+        for (int q = 0; q < 32; q += 2 * sft) e[q] = e[q] + e[q + sft];
+    const double t = lane_pairwise32(e[0]);
+    if (lane == 0) leaves[g] = t;
+}
+
 int launch_det_sum(const DetInput &in, double *chunk_tmp, double *out, cudaStream_t st) {
+    if (in.n > 0 && in.n <= kDetWarp * kDetSmemLeaves) {
+        const uint64_t G = (in.n + kDetWarp - 1) / kDetWarp;
+        uint64_t P = 1;
+        while (P < G) P <<= 1;
+        k_det_warps<<<unsigned((G + 1) / 2), 64, 0, st>>>(in, chunk_tmp + P, G), note_launch();
+        k_det_final<<<1, kDetThreads, 0, st>>>(chunk_tmp, P, G, out), note_launch();
+        MC_CUDA_TRY(cudaGetLastError());
+        return MC_OK;
+    }
     const uint64_t G = det_chunks(in.n), P = det_leaves(in.n);
     if (G == 0) {
         MC_CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(double), st));
@@ -434,7 +468,7 @@ int launch_row_sums_csr(const float *vals, const uint64_t *indptr, uint64_t n, u
 // ------------------------------------------------------------------------------------
 // Stable counting sort of rows by cluster id.
 // keys[i] in [0,k); optional keys2[i] (second membership, 0xffffffff = none).
-// Tiles of kSortTile rows; per-tile counts (key-major: tile_counts[key][tile]) -> per
+// Tiles of 512 or kSortTile rows; per-tile counts (key-major: tile_counts[key][tile]) -> per
 // (key, tile) offsets by a parallel scan per key -> one warp per tile scatters its rows in
 // order (match_any ranks), so each bucket lists rows ascending.
 // ------------------------------------------------------------------------------------
@@ -442,10 +476,11 @@ int launch_row_sums_csr(const float *vals, const uint64_t *indptr, uint64_t n, u
 constexpr uint32_t kSmemKeys = 8192;
 
 __global__ void k_sort_count(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ keys2, uint64_t n,
-                             uint32_t k, uint64_t ntiles, uint32_t *tile_counts /* [k][ntiles] */) {
+                             uint32_t k, uint64_t ntiles, uint64_t tile_rows,
+                             uint32_t *tile_counts /* [k][ntiles] */) {
     __shared__ uint32_t hist[kSmemKeys];
     const uint64_t tile = blockIdx.x;
-    const uint64_t b = tile * kSortTile, e = umin64(n, b + kSortTile);
+    const uint64_t b = tile * tile_rows, e = umin64(n, b + tile_rows);
     const bool sm = k <= kSmemKeys;
     if (sm) {
         for (uint32_t j = threadIdx.x; j < k; j += blockDim.x) hist[j] = 0;
@@ -541,7 +576,7 @@ __global__ void __launch_bounds__(1024) k_exclusive_scan_u64(const uint64_t *in,
 }
 
 __global__ void k_sort_scatter(const uint32_t *__restrict__ keys, uint64_t n, uint32_t k, uint64_t ntiles,
-                               uint32_t *tile_offsets, const uint64_t *__restrict__ bucket_start, uint32_t *perm) {
+                               uint64_t tile_rows, uint32_t *tile_offsets, const uint64_t *__restrict__ bucket_start, uint32_t *perm) {
     // one warp per tile; rows in order, 32 at a time; ranks from match_any.  Cursors live in
     // dynamic shared memory sized to k when k <= kSmemKeys (so that many one-warp blocks fit
     // on an SM), else in the tile's column of tile_offsets (stride ntiles).  The keys of 16
@@ -549,9 +584,9 @@ __global__ void k_sort_scatter(const uint32_t *__restrict__ keys, uint64_t n, ui
     extern __shared__ uint32_t scur[];
     const uint64_t tile = blockIdx.x;
     const int lane = threadIdx.x & 31;
-    const uint64_t b = tile * kSortTile;
+    const uint64_t b = tile * tile_rows;
     if (b >= n) return;
-    const uint64_t e = umin64(n, b + kSortTile);
+    const uint64_t e = umin64(n, b + tile_rows);
     const bool sm = k <= kSmemKeys;
     if (sm) {
         for (uint32_t j = lane; j < k; j += 32) scur[j] = tile_offsets[uint64_t(j) * ntiles + tile];
@@ -590,12 +625,12 @@ __global__ void k_sort_scatter(const uint32_t *__restrict__ keys, uint64_t n, ui
 // Rare path (rows with a second membership after an empty-cluster restart): one thread
 // per tile walks its rows in order so that every bucket stays ascending.
 __global__ void k_sort_scatter2(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ keys2, uint64_t n,
-                                uint32_t k, uint64_t ntiles, uint32_t *tile_offsets,
+                                uint32_t k, uint64_t ntiles, uint64_t tile_rows, uint32_t *tile_offsets,
                                 const uint64_t *__restrict__ bucket_start, uint32_t *perm) {
     const uint64_t tile = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
-    const uint64_t b = tile * kSortTile;
+    const uint64_t b = tile * tile_rows;
     if (b >= n) return;
-    const uint64_t e = umin64(n, b + kSortTile);
+    const uint64_t e = umin64(n, b + tile_rows);
     uint32_t *cur = tile_offsets + tile;
     for (uint64_t i = b; i < e; ++i) {
         const uint32_t k1 = keys[i], k2 = keys2[i];
@@ -673,16 +708,24 @@ int launch_exclusive_scan_u64(const uint64_t *in, uint64_t *out, uint64_t m, cud
     return MC_OK;
 }
 
+// Rows per sort tile (any size gives the same permutation).  A tile's rows are scattered by one
+// warp, 32 after 32, so short tiles finish sooner (10,000 rows: 15.4 -> 5 us with 512 rows); every
+// tile costs k counts, written, scanned and read, so long lists and many keys keep 2048.
+static uint64_t sort_tile_rows(uint64_t n, uint32_t k) {
+    return n <= (1u << 19) && uint64_t(k) * (n / 512) <= (1u << 19) ? 512 : kSortTile;
+}
+
 int launch_sort_by_key(const uint32_t *keys, const uint32_t *keys2, uint64_t n, uint32_t k, SortWork &w,
                        cudaStream_t st) {
-    const uint64_t ntiles = (n + kSortTile - 1) / kSortTile;
+    const uint64_t tile_rows = sort_tile_rows(n, k);
+    const uint64_t ntiles = (n + tile_rows - 1) / tile_rows;
     MC_TRY(w.tile_counts.alloc(ntiles * k, st));
     MC_TRY(w.bucket_count.alloc(k, st));
     MC_TRY(w.bucket_start.alloc(uint64_t(k) + 1, st));
     MC_TRY(w.perm.alloc(keys2 ? 2 * n : n, st));
     if (k > kSmemKeys) MC_CUDA_TRY(cudaMemsetAsync(w.tile_counts.p, 0, ntiles * k * sizeof(uint32_t), st));
     if (ntiles)
-        k_sort_count<<<unsigned(ntiles), 256, 0, st>>>(keys, keys2, n, k, ntiles, w.tile_counts.p), note_launch();
+        k_sort_count<<<unsigned(ntiles), 256, 0, st>>>(keys, keys2, n, k, ntiles, tile_rows, w.tile_counts.p), note_launch();
     else
         MC_CUDA_TRY(cudaMemsetAsync(w.bucket_count.p, 0, k * sizeof(uint64_t), st));
     if (ntiles) k_sort_key_scan<<<k, 256, 0, st>>>(w.tile_counts.p, ntiles, k, w.bucket_count.p), note_launch();
@@ -690,11 +733,11 @@ int launch_sort_by_key(const uint32_t *keys, const uint32_t *keys2, uint64_t n, 
     if (ntiles) {
         if (!keys2)
             k_sort_scatter<<<unsigned(ntiles), 32, k <= kSmemKeys ? k * sizeof(uint32_t) : 0, st>>>(
-                keys, n, k, ntiles, w.tile_counts.p, w.bucket_start.p,
+                keys, n, k, ntiles, tile_rows, w.tile_counts.p, w.bucket_start.p,
                                                             w.perm.p), note_launch();
         else
             k_sort_scatter2<<<unsigned((ntiles + 63) / 64), 64, 0, st>>>(keys, keys2, n, k, ntiles,
-                                                                         w.tile_counts.p, w.bucket_start.p,
+                                                                         tile_rows, w.tile_counts.p, w.bucket_start.p,
                                                                          w.perm.p), note_launch();
     }
     MC_CUDA_TRY(cudaGetLastError());
@@ -706,64 +749,174 @@ int launch_sort_by_key(const uint32_t *keys, const uint32_t *keys2, uint64_t n, 
 // chunk_start[c] = exclusive scan of the chunk counts (computed on device); a grid of
 // ceil(n/ch)+k CTAs maps its chunk id by binary search, extra CTAs exit.
 // ------------------------------------------------------------------------------------
-// dense: one CTA per chunk (at most kDenseChunk rows of one cluster), threads over
-// columns, rows sequential.  The chunk's row ids are staged in shared memory and each
-// thread loads 8 rows' values ahead of its sequential sum, so the loads overlap.
+// dense: one warp per (chunk of at most kDenseChunk rows of one cluster, 32 V columns); lanes
+// hold V adjacent columns each, rows sequential.  The 32 row ids of a batch sit one per lane, and
+// eight rows are loaded while the eight before them are added, so a row costs a warp one
+// broadcast, one vector load and the seven adds of a TwoSum in packed f32x2 form (each half the
+// single operation).  Loads are unconditional (ids past the chunk are row 0): with a branch per
+// row they wait for one another (553 and 42 us in the two cases below).  4M x 128, k = 1024: 392 ->
+// 319 us (300 at the copy rate); 300,001 x 100, k = 200: 47 -> 28; 10,000 x 50, k = 25: 19.8 -> 11.5
+// (the round trips of 256 dependent rows).  Before: a thread per column, batches of eight.
 constexpr uint64_t kDenseChunk = 256;
 
-__global__ void __launch_bounds__(128) k_centroid_chunks_dense(const float *__restrict__ X, uint64_t d,
-                                                               const uint32_t *__restrict__ perm,
-                                                               const uint64_t *__restrict__ bucket_start,
-                                                               const uint64_t *__restrict__ bucket_count,
-                                                               const uint64_t *__restrict__ chunk_start, uint32_t k,
-                                                               uint64_t ch, const double *__restrict__ w,
-                                                               double *partial /* [chunk][d] */,
-                                                               double *partial_w /* [chunk] */) {
-    __shared__ uint32_t srows[kDenseChunk];
-    __shared__ double sw[kDenseChunk];
-    const uint64_t q = blockIdx.x;
-    if (q >= chunk_start[k]) return;
-    const uint32_t c = find_bucket(chunk_start, k, q);
-    const uint64_t local = q - chunk_start[c];
-    const uint64_t r0 = local * ch, r1 = umin64(bucket_count[c], r0 + ch);
-    const int cnt = int(r1 - r0);
-    const uint32_t *rows = perm + bucket_start[c] + r0;
-    for (int r = threadIdx.x; r < cnt; r += blockDim.x) {
-        srows[r] = rows[r];
-        if (w) sw[r] = w[rows[r]];
-    }
-    __syncthreads();
+__device__ __forceinline__ unsigned long long c2_add(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long c2_sub(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// two_sum_add in both halves
+__device__ __forceinline__ void c2_two_sum_add(unsigned long long &s, unsigned long long &e, unsigned long long x) {
+    const unsigned long long t = c2_add(s, x);
+    const unsigned long long bp = c2_sub(t, s);
+    const unsigned long long err = c2_add(c2_sub(s, c2_sub(t, bp)), c2_sub(x, bp));
+    s = t;
+    e = c2_add(e, err);
+}
+__device__ __forceinline__ void c2_unpack(unsigned long long v, float &lo, float &hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+
+template <int V>
+struct ColVec;
+template <>
+struct ColVec<1> {
+    using T = float;
+};
+template <>
+struct ColVec<2> {
+    using T = float2;
+};
+template <>
+struct ColVec<4> {
+    using T = float4;
+};
+
+template <int V, bool WEIGHTED>
+__global__ void __launch_bounds__(128) k_centroid_rows_dense(const float *__restrict__ X, uint64_t d, uint32_t slices,
+                                                             const uint32_t *__restrict__ perm,
+                                                             const uint64_t *__restrict__ bucket_start,
+                                                             const uint64_t *__restrict__ bucket_count,
+                                                             const uint64_t *__restrict__ chunk_start, uint32_t k,
+                                                             uint64_t ch, const double *__restrict__ w,
+                                                             double *partial /* [chunk][d] */,
+                                                             double *partial_w /* [chunk] */) {
+    using T = typename ColVec<V>::T;
     constexpr int U = 8;
-    for (uint64_t j = threadIdx.x; j < d; j += blockDim.x) {
-        if (w) {
-            double acc = 0.0;
-            for (int r = 0; r < cnt; r += U) {
-                float xv[U];
+    const int lane = threadIdx.x & 31;
+    const uint64_t task = blockIdx.x * uint64_t(4) + (threadIdx.x >> 5);
+    const uint64_t q = task / slices;
+    const uint32_t slice = uint32_t(task - q * slices);
+    if (q >= chunk_start[k]) return;  // whole warp; no block barrier
+    const uint32_t c = find_bucket(chunk_start, k, q);
+    const uint64_t r0 = (q - chunk_start[c]) * ch;
+    const int cnt = int(umin64(bucket_count[c] - r0, ch));
+    const uint32_t *rows = perm + bucket_start[c] + r0;
+    const uint64_t j = uint64_t(slice) * 32 * V + uint64_t(lane) * V;
+    const bool on = j < d;  // d % V == 0
+    const float *Xj = X + (on ? j : 0);
+    // row ids (and weights) of the 32 rows at hand and the next 32; past the chunk: row 0, unused
+    uint32_t id = lane < cnt ? rows[lane] : 0u, idn = 32 + lane < cnt ? rows[32 + lane] : 0u;
+    double wt = 0.0, wtn = 0.0;
+    if (WEIGHTED) {
+        wt = lane < cnt ? w[id] : 0.0;
+        wtn = 32 + lane < cnt ? w[idn] : 0.0;
+    }
+    T xa[U], xb[U];
+    // rows rel .. rel + U - 1 past the batch's first row (unconditional: ids past the chunk are 0)
+    auto load = [&](int rel, T (&x)[U]) {
 #pragma unroll
-                for (int u = 0; u < U; ++u) xv[u] = (r + u < cnt) ? X[uint64_t(srows[r + u]) * d + j] : 0.f;
+        for (int u = 0; u < U; ++u) {
+            const uint32_t row = __shfl_sync(0xffffffffu, rel + u < 32 ? id : idn, (rel + u) & 31);
+            x[u] = __ldg(reinterpret_cast<const T *>(Xj + uint64_t(row) * d));
+        }
+    };
+    float s1 = 0.f, e1 = 0.f;
+    unsigned long long s[V / 2 ? V / 2 : 1] = {}, e[V / 2 ? V / 2 : 1] = {};
+    double acc[V] = {}, wq = 0.0;
+    auto add_row = [&](int rel, const T &xr) {
+        const float *f = reinterpret_cast<const float *>(&xr);
+        if (WEIGHTED) {
+            const double sw = __shfl_sync(0xffffffffu, wt, rel & 31);
 #pragma unroll
-                for (int u = 0; u < U; ++u)
-                    if (r + u < cnt) acc = fma(sw[r + u], double(xv[u]), acc);
-            }
-            partial[q * d + j] = acc;
+            for (int v = 0; v < V; ++v) acc[v] = fma(sw, double(f[v]), acc[v]);
+            if (slice == 0) wq = wq + sw;
+        } else if (V == 1) {
+            two_sum_add(s1, e1, f[0]);
         } else {
-            float s = 0.f, e = 0.f;
-            for (int r = 0; r < cnt; r += U) {
-                float xv[U];
+            const unsigned long long *f2 = reinterpret_cast<const unsigned long long *>(&xr);
 #pragma unroll
-                for (int u = 0; u < U; ++u) xv[u] = (r + u < cnt) ? X[uint64_t(srows[r + u]) * d + j] : 0.f;
+            for (int v = 0; v < V / 2; ++v) c2_two_sum_add(s[v], e[v], f2[v]);
+        }
+    };
+    auto add = [&](int rel, const T (&x)[U]) {
 #pragma unroll
-                for (int u = 0; u < U; ++u)
-                    if (r + u < cnt) two_sum_add(s, e, xv[u]);
-            }
-            partial[q * d + j] = double(s) + double(e);
+        for (int u = 0; u < U; ++u) add_row(rel + u, x[u]);
+    };
+    auto add_some = [&](int rel, int left, const T (&x)[U]) {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (rel + u < left) add_row(rel + u, x[u]);  // warp-uniform
+    };
+    load(0, xa);
+    load(8, xb);
+    for (int rb = 0; rb < cnt; rb += 32) {
+        const int left = cnt - rb;
+        if (left >= 32) {
+            add(0, xa);
+            load(16, xa);
+            add(8, xb);
+            load(24, xb);
+            add(16, xa);
+            load(32, xa);
+            add(24, xb);
+            load(40, xb);
+        } else {
+            add_some(0, left, xa);
+            load(16, xa);
+            add_some(8, left, xb);
+            load(24, xb);
+            add_some(16, left, xa);
+            add_some(24, left, xb);
+        }
+        id = idn;
+        wt = wtn;
+        idn = rb + 64 + lane < cnt ? rows[rb + 64 + lane] : 0u;
+        if (WEIGHTED) wtn = rb + 64 + lane < cnt ? w[idn] : 0.0;
+    }
+    if (WEIGHTED && slice == 0 && lane == 0) partial_w[q] = wq;
+    if (!on) return;
+    double *out = partial + q * d + j;
+    if (WEIGHTED) {
+#pragma unroll
+        for (int v = 0; v < V; ++v) out[v] = acc[v];
+    } else if (V == 1) {
+        out[0] = double(s1) + double(e1);
+    } else {
+#pragma unroll
+        for (int v = 0; v < V / 2; ++v) {
+            float sl, sh, el, eh;
+            c2_unpack(s[v], sl, sh);
+            c2_unpack(e[v], el, eh);
+            out[2 * v] = double(sl) + double(el);
+            out[2 * v + 1] = double(sh) + double(eh);
         }
     }
-    if (w && threadIdx.x == 0) {
-        double wq = 0.0;
-        for (int r = 0; r < cnt; ++r) wq = wq + sw[r];
-        partial_w[q] = wq;
-    }
+}
+
+template <int V>
+static int centroid_rows_dense(const CentroidArgs &a, SortWork &w, uint64_t max_chunks, uint64_t ch, cudaStream_t st) {
+    const uint32_t slices = uint32_t((a.d + 32 * V - 1) / (32 * V));
+    auto kern = a.w ? k_centroid_rows_dense<V, true> : k_centroid_rows_dense<V, false>;
+    kern<<<unsigned((max_chunks * slices + 3) / 4), 128, 0, st>>>(
+        a.X, a.d, slices, w.perm.p, w.bucket_start.p, w.bucket_count.p, w.chunk_start.p, a.k, ch, a.w, w.partial.p,
+        w.partial_w.p), note_launch();
+    MC_CUDA_TRY(cudaGetLastError());
+    return MC_OK;
 }
 
 // CSR: one CTA per (chunk, column band); dense band accumulator in shared memory.
@@ -1002,9 +1155,11 @@ int launch_centroids(const CentroidArgs &a, SortWork &w, cudaStream_t st, bool p
     MC_TRY(w.partial.alloc(max_chunks * d, st));
     MC_TRY(w.partial_w.alloc(max_chunks, st));
     if (!a.csr) {
-        k_centroid_chunks_dense<<<unsigned(max_chunks), 128, 0, st>>>(a.X, d, w.perm.p, w.bucket_start.p,
-                                                                     w.bucket_count.p, w.chunk_start.p, k, ch, a.w,
-                                                                     w.partial.p, w.partial_w.p), note_launch();
+        // the widest columns per lane that still give every lane some
+        const uintptr_t xp = reinterpret_cast<uintptr_t>(a.X);
+        if (d >= 96 && d % 4 == 0 && xp % 16 == 0) MC_TRY(centroid_rows_dense<4>(a, w, max_chunks, ch, st));
+        else if (d >= 48 && d % 2 == 0 && xp % 8 == 0) MC_TRY(centroid_rows_dense<2>(a, w, max_chunks, ch, st));
+        else MC_TRY(centroid_rows_dense<1>(a, w, max_chunks, ch, st));
     } else {
         bool done = false;
         MC_TRY(launch_centroid_chunks_csr(a, w, max_chunks, ch, st, &done));
