@@ -122,9 +122,29 @@ __global__ void k_cluster_partials(const double *__restrict__ vals, const uint32
     const uint32_t c = lo;
     const uint64_t r0 = (q - chunk_start[c]) * 256, r1 = umin64(bucket_count[c], r0 + 256);
     const uint32_t *rows = perm + bucket_start[c];
+    // 16 row ids, then their 16 values in flight before the adds (in order); past the chunk its
+    // last row, not added: loads under a condition would wait for one another
     double p = 0.0;
-    for (uint64_t r = r0; r < r1; ++r) p = p + vals[rows[r]];
+    for (uint64_t r = r0; r < r1; r += 16) {
+        uint32_t id[16];
+        double v[16];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) id[u] = rows[r + u < r1 ? r + u : r1 - 1];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) v[u] = vals[id[u]];
+#pragma unroll
+        for (int u = 0; u < 16; ++u)
+            if (r + u < r1) p = p + v[u];
+    }
     partial[q] = p;
+}
+
+// sums of ones: the counts
+__global__ void k_cluster_counts(const uint64_t *bucket_count, uint32_t k, double *a, double *b) {
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= k) return;
+    a[c] = double(bucket_count[c]);
+    if (b) b[c] = double(bucket_count[c]);
 }
 
 __global__ void k_cluster_final(const double *partial, const uint64_t *chunk_start, uint32_t k, double *out) {
@@ -155,6 +175,7 @@ struct SensArgs {
     const double *total;   // device scalar: total (w * cost) or (w * cost^2) for LFKF
     double alpha, alpha_est;
     const double *W;       // LBK: sum of weight sums (device scalar)
+    double *adj;           // LBK: [nc] the cluster's addend (k_lbk_adj); [nc] the cost's factor at adj[nc]
     double *s;
     float *probs;          // FL writes probs directly
 };
@@ -163,6 +184,17 @@ __global__ void k_lbk_W(const double *wsum, uint32_t nc, double *W) {
     double s = 0.0;
     for (uint32_t c = 0; c < nc; ++c) s = s + wsum[c];
     *W = s;
+}
+
+// LBK: what a point's sensitivity takes from its cluster, once per cluster (two FP64 divisions per
+// point took 150 us at 2M points; about two FP64 lane operations fit an SM's clock)
+__global__ void k_lbk_adj(SensArgs a) {
+    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g > a.nc) return;
+    const double W = *a.W;
+    const double avg = *a.total / W;
+    a.adj[g] = g == a.nc ? a.alpha / avg
+                         : (2.0 * a.alpha) * a.csum[g] / (a.wsum[g] * avg) + 4.0 * W / a.wsum[g];
 }
 
 __global__ void k_sens(SensArgs a) {
@@ -191,23 +223,24 @@ __global__ void k_sens(SensArgs a) {
                 a.s[i] = w * c / total + 1.0 / a.cnt[g];
                 break;
             default: {  // LBK
-                const double W = *a.W;
-                const double avg = total / W;
-                const double tcinv = a.alpha / avg;
-                const double adj = (2.0 * a.alpha) * a.csum[g] / (a.wsum[g] * avg) + 4.0 * W / a.wsum[g];
-                a.s[i] = tcinv * c + adj;
+                a.s[i] = a.adj[a.nc] * c + a.adj[g];
             }
         }
     }
 }
 
 __global__ void k_normalize(const double *s, uint64_t n, const double *tot, float *probs) {
-    const double inv = 1.0 / *tot;
+    __shared__ double sm_inv;  // one FP64 division per CTA
+    if (threadIdx.x == 0) sm_inv = 1.0 / *tot;
+    __syncthreads();
+    const double inv = sm_inv;
     for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n; i += gridDim.x * uint64_t(blockDim.x))
         probs[i] = float(s[i] * inv);
 }
 
 static unsigned grid_for(uint64_t n, int sms) { return unsigned(umin64((n + 255) / 256, uint64_t(sms) * 32)) + 1; }
+// kernels that start with an FP64 division per CTA: one wave
+static unsigned grid_wave(uint64_t n, int sms) { return unsigned(umin64((n + 255) / 256, uint64_t(sms) * 8)) + 1; }
 
 int compute_sensitivities(const SensInput &in, SensWork &w, cudaStream_t st, int sms) {
     const uint64_t n = in.n;
@@ -217,6 +250,7 @@ int compute_sensitivities(const SensInput &in, SensWork &w, cudaStream_t st, int
     MC_TRY(w.cnt.alloc(nc, st));
     MC_TRY(w.wsum.alloc(nc, st));
     MC_TRY(w.csum.alloc(nc, st));
+    MC_TRY(w.adj.alloc(uint64_t(nc) + 1, st));
     MC_TRY(w.scal.alloc(4, st));
     MC_TRY(w.det_tmp.alloc(det_tmp_size(n), st));
     MC_TRY(w.flag.alloc(1, st));
@@ -235,21 +269,29 @@ int compute_sensitivities(const SensInput &in, SensWork &w, cudaStream_t st, int
     const uint64_t maxq = (n + 255) / 256 + nc;
     MC_TRY(w.sort.partial.alloc(maxq, st));
     auto cluster_sum = [&](int kind, double *out) -> int {
-        k_point_vals<<<grid_for(n, sms), 256, 0, st>>>(in.cost, in.wt, n, kind, w.vals.p), note_launch();
-        k_cluster_partials<<<unsigned((maxq + 255) / 256), 256, 0, st>>>(w.vals.p, w.sort.perm.p, w.sort.bucket_start.p,
+        // the cost itself is the value where there are no weights (kind 2: 1.0 * cost)
+        const double *vals = in.cost;
+        if (in.wt || kind != 2) {
+            k_point_vals<<<grid_for(n, sms), 256, 0, st>>>(in.cost, in.wt, n, kind, w.vals.p), note_launch();
+            vals = w.vals.p;
+        }
+        k_cluster_partials<<<unsigned((maxq + 63) / 64), 64, 0, st>>>(vals, w.sort.perm.p, w.sort.bucket_start.p,
                                                                         w.sort.bucket_count.p, w.sort.chunk_start.p, nc,
                                                                         w.sort.partial.p), note_launch();
         k_cluster_final<<<(nc + 255) / 256, 256, 0, st>>>(w.sort.partial.p, w.sort.chunk_start.p, nc, out), note_launch();
         MC_CUDA_TRY(cudaGetLastError());
         return MC_OK;
     };
-    MC_TRY(cluster_sum(0, w.cnt.p));
-    MC_TRY(cluster_sum(1, w.wsum.p));
+    // sums of ones are the counts, exactly
+    k_cluster_counts<<<(nc + 255) / 256, 256, 0, st>>>(w.sort.bucket_count.p, nc, w.cnt.p, in.wt ? nullptr : w.wsum.p),
+        note_launch();
+    if (in.wt) MC_TRY(cluster_sum(1, w.wsum.p));
     const int tkind = in.method == MC_LFKF ? 3 : 2;
     if (in.method == MC_LBK || in.method == MC_LFKF) MC_TRY(cluster_sum(tkind, w.csum.p));
     // total (w*cost, or w*cost^2 for LFKF) in the canonical det order
-    k_point_vals<<<grid_for(n, sms), 256, 0, st>>>(in.cost, in.wt, n, tkind, w.vals.p), note_launch();
-    DetInput di{DET_F64, w.vals.p, nullptr, nullptr, n};
+    if (in.wt || tkind != 2)
+        k_point_vals<<<grid_for(n, sms), 256, 0, st>>>(in.cost, in.wt, n, tkind, w.vals.p), note_launch();
+    DetInput di{DET_F64, in.wt || tkind != 2 ? w.vals.p : in.cost, nullptr, nullptr, n};
     MC_TRY(launch_det_sum(di, w.det_tmp.p, w.scal.p + 0, st));
     if (in.method == MC_LBK) k_lbk_W<<<1, 1, 0, st>>>(w.wsum.p, nc, w.scal.p + 1), note_launch();
     SensArgs sa;
@@ -266,13 +308,15 @@ int compute_sensitivities(const SensInput &in, SensWork &w, cudaStream_t st, int
     sa.alpha = 16.0 * log(double(in.k)) + 32.0;
     sa.alpha_est = in.alpha_est;
     sa.W = w.scal.p + 1;
+    sa.adj = w.adj.p;
     sa.s = w.s.p;
     sa.probs = in.probs;
+    if (in.method == MC_LBK) k_lbk_adj<<<(nc + 256) / 256, 256, 0, st>>>(sa), note_launch();
     k_sens<<<grid_for(n, sms), 256, 0, st>>>(sa), note_launch();
     if (in.method != MC_FL) {
         DetInput ds{DET_F64, w.s.p, nullptr, nullptr, n};
         MC_TRY(launch_det_sum(ds, w.det_tmp.p, w.scal.p + 2, st));
-        k_normalize<<<grid_for(n, sms), 256, 0, st>>>(w.s.p, n, w.scal.p + 2, in.probs), note_launch();
+        k_normalize<<<grid_wave(n, sms), 256, 0, st>>>(w.s.p, n, w.scal.p + 2, in.probs), note_launch();
     }
     MC_CUDA_TRY(cudaGetLastError());
     return MC_OK;
@@ -281,15 +325,27 @@ int compute_sensitivities(const SensInput &in, SensWork &w, cudaStream_t st, int
 // ------------------------------------------------------------------------------------
 // alias table
 // ------------------------------------------------------------------------------------
+// n / S, one FP64 division per CTA (a division per thread took most of these kernels' time)
+__device__ __forceinline__ double alias_scale(uint64_t n, const double *S) {
+    __shared__ double sm_scale;
+    if (threadIdx.x == 0) sm_scale = double(n) / *S;
+    __syncthreads();
+    return sm_scale;
+}
+
+// a < b for values that are not negative (nor NaN): their bits as integers, because FP64
+// comparisons run at about two lanes per SM and clock
+__device__ __forceinline__ bool nn_less(double a, double b) { return __double_as_longlong(a) < __double_as_longlong(b); }
+
 __global__ void k_alias_flags(const float *probs, uint64_t n, const double *S, uint64_t *light_flag) {
-    const double scale = double(n) / *S;
+    const double scale = alias_scale(n, S);
     for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n; i += gridDim.x * uint64_t(blockDim.x))
         light_flag[i] = (double(probs[i]) * scale < 1.0) ? 1 : 0;
 }
 
 __global__ void k_alias_lists(const float *probs, uint64_t n, const double *S, const uint64_t *light_pos,
                               uint32_t *L, uint32_t *H, double *dl, double *eh) {
-    const double scale = double(n) / *S;
+    const double scale = alias_scale(n, S);
     for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n; i += gridDim.x * uint64_t(blockDim.x)) {
         const double q = double(probs[i]) * scale;
         const uint64_t lp = light_pos[i];
@@ -307,13 +363,13 @@ __global__ void k_alias_lists(const float *probs, uint64_t n, const double *S, c
 __global__ void k_alias_light(const float *probs, uint64_t n, const double *S, const uint32_t *L, uint64_t nl,
                               const uint32_t *H, uint64_t nh, const double *D, const double *E, double *prob_tab,
                               uint32_t *alias_tab) {
-    const double scale = double(n) / *S;
+    const double scale = alias_scale(n, S);
     for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < nl; i += gridDim.x * uint64_t(blockDim.x)) {
         const double Di = D[i];
         uint64_t lo = 0, hi = nh;
         while (lo < hi) {
             const uint64_t mid = (lo + hi) >> 1;
-            if (E[mid + 1] >= Di) hi = mid; else lo = mid + 1;
+            if (nn_less(E[mid + 1], Di)) lo = mid + 1; else hi = mid;
         }
         const uint64_t j = lo < nh ? lo : nh - 1;
         const uint32_t li = L[i];
@@ -331,7 +387,7 @@ __global__ void k_alias_heavy(const uint32_t *H, uint64_t nh, uint64_t nl, const
             uint64_t lo = 0, hi = nl;
             while (lo < hi) {
                 const uint64_t mid = (lo + hi) >> 1;
-                if (D[mid + 1] > Ej) hi = mid; else lo = mid + 1;
+                if (nn_less(Ej, D[mid + 1])) hi = mid; else lo = mid + 1;
             }
             i = lo;
         }
@@ -371,7 +427,7 @@ int build_alias(const float *probs, uint64_t n, double *prob_tab, uint32_t *alia
     MC_CUDA_TRY(cudaMemcpyAsync(&S, w.S.p, sizeof(double), cudaMemcpyDeviceToHost, st));
     MC_CUDA_TRY(cudaStreamSynchronize(st));
     if (!(S > 0.0)) return fail(MC_EINVAL, "sampling probabilities sum to a non-positive value");
-    k_alias_flags<<<grid_for(n, sms), 256, 0, st>>>(probs, n, w.S.p, w.flag.p), note_launch();
+    k_alias_flags<<<grid_wave(n, sms), 256, 0, st>>>(probs, n, w.S.p, w.flag.p), note_launch();
     MC_TRY(launch_exclusive_scan_u64(w.flag.p, w.pos.p, n, st));
     uint64_t nl = 0;
     MC_CUDA_TRY(cudaMemcpyAsync(&nl, w.pos.p + n, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
@@ -382,10 +438,10 @@ int build_alias(const float *probs, uint64_t n, double *prob_tab, uint32_t *alia
         MC_CUDA_TRY(cudaGetLastError());
         return MC_OK;
     }
-    k_alias_lists<<<grid_for(n, sms), 256, 0, st>>>(probs, n, w.S.p, w.pos.p, w.L.p, w.H.p, w.dl.p, w.eh.p), note_launch();
+    k_alias_lists<<<grid_wave(n, sms), 256, 0, st>>>(probs, n, w.S.p, w.pos.p, w.L.p, w.H.p, w.dl.p, w.eh.p), note_launch();
     MC_TRY(canon_exclusive_scan(w.dl.p, nl, w.D.p, w.scan, st));
     MC_TRY(canon_exclusive_scan(w.eh.p, nh, w.E.p, w.scan, st));
-    if (nl) k_alias_light<<<grid_for(nl, sms), 256, 0, st>>>(probs, n, w.S.p, w.L.p, nl, w.H.p, nh, w.D.p, w.E.p,
+    if (nl) k_alias_light<<<grid_wave(nl, sms), 256, 0, st>>>(probs, n, w.S.p, w.L.p, nl, w.H.p, nh, w.D.p, w.E.p,
                                                              prob_tab, alias_tab), note_launch();
     k_alias_heavy<<<grid_for(nh, sms), 256, 0, st>>>(w.H.p, nh, nl, w.D.p, w.E.p, prob_tab, alias_tab), note_launch();
     MC_CUDA_TRY(cudaGetLastError());

@@ -22,7 +22,7 @@ struct SensInput {
 };
 
 struct SensWork {
-    DBuf<double> vals, s, cnt, wsum, csum, scal, det_tmp;
+    DBuf<double> vals, s, cnt, wsum, csum, adj, scal, det_tmp;
     DBuf<int> flag;
     SortWork sort;
 };
