@@ -759,28 +759,6 @@ int launch_sort_by_key(const uint32_t *keys, const uint32_t *keys2, uint64_t n, 
 // (the round trips of 256 dependent rows).  Before: a thread per column, batches of eight.
 constexpr uint64_t kDenseChunk = 256;
 
-__device__ __forceinline__ unsigned long long c2_add(unsigned long long a, unsigned long long b) {
-    unsigned long long r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ unsigned long long c2_sub(unsigned long long a, unsigned long long b) {
-    unsigned long long r;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-// two_sum_add in both halves
-__device__ __forceinline__ void c2_two_sum_add(unsigned long long &s, unsigned long long &e, unsigned long long x) {
-    const unsigned long long t = c2_add(s, x);
-    const unsigned long long bp = c2_sub(t, s);
-    const unsigned long long err = c2_add(c2_sub(s, c2_sub(t, bp)), c2_sub(x, bp));
-    s = t;
-    e = c2_add(e, err);
-}
-__device__ __forceinline__ void c2_unpack(unsigned long long v, float &lo, float &hi) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-
 template <int V>
 struct ColVec;
 template <>

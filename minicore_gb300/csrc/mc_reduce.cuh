@@ -55,6 +55,39 @@ __device__ inline void two_sum_add(float &s, float &e, float x) {
     e = __fadd_rn(e, err);
 }
 
+// packed f32x2: each half is the IEEE single operation
+__device__ __forceinline__ unsigned long long c2_add(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long c2_sub(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// two_sum_add in both halves
+__device__ __forceinline__ void c2_two_sum_add(unsigned long long &s, unsigned long long &e, unsigned long long x) {
+    const unsigned long long t = c2_add(s, x);
+    const unsigned long long bp = c2_sub(t, s);
+    const unsigned long long err = c2_add(c2_sub(s, c2_sub(t, bp)), c2_sub(x, bp));
+    s = t;
+    e = c2_add(e, err);
+}
+__device__ __forceinline__ void c2_unpack(unsigned long long v, float &lo, float &hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long c2_mul(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long c2_pack(float lo, float hi) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+
 int launch_sort_by_key(const uint32_t *keys, const uint32_t *keys2, uint64_t n, uint32_t k, SortWork &w,
                        cudaStream_t st);
 // chunk partials over CSR rows (mc_centroid_csr.cu); *done = false: not covered there
