@@ -273,6 +273,7 @@ struct mc_job {
     uint32_t ngrp = 0;
     SortWork sort;
     L1CsrWork l1csr;  // L1 medians over CSR rows
+    DBuf<L1Stat> l1stat;  // dense L1 in pair mode: the rows' part is written at creation
     DBuf<float> clist;  // L1 pair-mode CSR assignment: per 32-center group, columns and values
     TcState tc;
     uint64_t last_recheck = 0;
@@ -408,6 +409,10 @@ int job_assign_with(mc_job *j, const float *C, double prior_sum, bool force_exac
         a.consts = j->consts.p;
     }
     MC_TRY(launch_prep_centers(a, C, j->pair, sparse, j->st));
+    if (j->l1stat.p) {
+        MC_TRY(launch_l1_center_stat(C, uint64_t(j->k) * d, j->csum.p, j->k, j->l1stat.p, j->st));
+        a.l1 = j->l1stat.p;
+    }
     if (sparse && j->msr == JSD) {
         MC_TRY(j->ztab.alloc(uint64_t(j->ngrp) * j->k, j->st));
         MC_TRY(launch_jsd_ztable(C, j->k, d, j->csum.p, j->pv, j->gval.p, j->ngrp, j->ztab.p, j->st));
@@ -484,7 +489,7 @@ int job_l1_medians(mc_job *j) {
     Phase ph("centroid_update", j->st);
     MC_CUDA_TRY(cudaMemsetAsync(j->flag.p, 0, sizeof(int), j->st));
     if (j->M.kind == MC_DENSE_F32)
-        return launch_l1_medians(j->M.X, j->M.d, j->k, j->sort, j->w.p, j->Cw.p, j->st);
+        return launch_l1_medians(j->M.X, j->M.n, j->M.d, j->k, j->sort, j->w.p, j->Cw.p, j->st);
     // the reference's CSR median takes no weights (util/csc.h:835)
     if (j->w.p) return fail(MC_EUNSUPPORTED, "Not implemented: weighted L1 median for CSparseMatrix");
     return launch_l1_medians_csr(j->M.vals, j->M.idx, j->M.indptr, j->M.n, j->M.d, j->M.nnz, j->k, j->asn.p,
@@ -1036,14 +1041,9 @@ __global__ void k_soft_rows(const float *__restrict__ costs, uint64_t n, uint32_
     rowval[i] = double(dot);
 }
 
-// soft weighted means in two steps with the order of a sequential walk: per chunk of 256
-// rows and center c, thread j keeps a compensated float sum of coef * x[r][j] (coef = asn *
-// float(w)) and of coef; then per (c, j) the chunk values are added in FP64 in chunk order,
-// and center = num * (1 / den)
-constexpr uint64_t kSoftChunk = 256;
 // The same with the rows' costs and assignments in shared memory (row pitch odd: a thread walks
 // its row without bank conflicts), copied in and out coalesced.  A thread per row straight from
-// memory touches 32 rows per load: 200,000 x 20: 103 -> 30 us.
+// memory touches 32 rows per load: 200,000 x 20: 103 -> 27 us.
 __global__ void __launch_bounds__(128) k_soft_rows_staged(const float *__restrict__ costs, uint64_t n, uint32_t k,
                                                           float temp, float *__restrict__ asn,
                                                           double *__restrict__ rowval) {
@@ -1100,11 +1100,16 @@ static int launch_soft_rows(const float *costs, uint64_t n, uint32_t k, float te
     return MC_OK;
 }
 
+// soft weighted means in two steps with the order of a sequential walk: per chunk of 256
+// rows and center c, thread j keeps a compensated float sum of coef * x[r][j] (coef = asn *
+// float(w)) and of coef; then per (c, j) the chunk values are added in FP64 in chunk order,
+// and center = num * (1 / den)
+constexpr uint64_t kSoftChunk = 256;
 
 // One CTA per (chunk, 32 columns, 32 centers): the chunk's columns and coefficients in shared
 // memory once for all its centers, lane = column, warp w = centers 4w .. 4w + 3 as two packed
 // f32x2 TwoSums (a CTA per (chunk, center) read the rows again for every center, one dependent
-// row after the other: 200,000 x 32, k = 20: 133 -> 45 us).
+// row after the other: 200,000 x 32, k = 20: 133 -> 65 us).
 __global__ void __launch_bounds__(256) k_soft_center_chunks(const float *__restrict__ X, uint64_t n, uint64_t d,
                                                             const float *__restrict__ asn, uint32_t k,
                                                             const double *__restrict__ w,
@@ -1234,7 +1239,7 @@ __global__ void __launch_bounds__(256) k_soft_l1_centers(const float *__restrict
 
 // Adds the partials of chunks [0, nq) of one batch to the running FP64 sums: 16 runs of
 // consecutive chunks in order, the run sums as a pairwise tree, then onto the running sum (one
-// chain over all chunks was 782 dependent loads and FP64 adds at 200,000 rows: 249 -> 12 us; the
+// chain over all chunks was 782 dependent loads and FP64 adds at 200,000 rows: 249 -> 23 us; the
 // tree's rounding error is no larger).
 constexpr int kSoftRuns = 16;
 
@@ -1531,6 +1536,10 @@ static int job_create_impl(mc_context *ctx, const mc_matrix *X, const float *cen
             MC_TRY(launch_row_scalars(j->rowsum.p, n, d, j->pv, j->rsi.p, j->rinc.p, st));
         }
     }
+    if (msr == L1 && j->pair && j->M.kind == MC_DENSE_F32) {
+        MC_TRY(j->l1stat.alloc(1, st));
+        MC_TRY(launch_l1_row_stat(j->M.X, n * d, j->rowsum.p, n, j->l1stat.p, st));
+    }
     j->sparse_path = j->M.kind == MC_CSR_F32 && !j->pair && (msr != JSD || j->ngrp > 0);
     *out = j.release();
     return MC_OK;
@@ -1745,7 +1754,7 @@ int mc_job_minibatch(mc_job *j, uint64_t mbsize, uint64_t maxiter, uint64_t calc
             // util/csc.h:829-893); groups without rows keep their center
             MC_TRY(launch_sort_by_key(sj->asn.p, nullptr, m, k, sj->sort, st));
             if (sj->M.kind == MC_DENSE_F32) {
-                MC_TRY(launch_l1_medians(sj->M.X, d, k, sj->sort, j->w.p, j->C.p, st, n));
+                MC_TRY(launch_l1_medians(sj->M.X, m, d, k, sj->sort, j->w.p, j->C.p, st, n));
             } else {
                 if (j->w.p) return fail(MC_EUNSUPPORTED, "Not implemented: weighted L1 median for CSparseMatrix");
                 MC_TRY(launch_l1_medians_csr(sj->M.vals, sj->M.idx, sj->M.indptr, m, d, sj->M.nnz, k, sj->asn.p,

@@ -209,6 +209,7 @@ __global__ void __launch_bounds__(256) k_assign_tiled(AssignArgs a) {
     const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
     const uint64_t row0 = uint64_t(blockIdx.x) * BM;
     const uint64_t d = a.d;
+    if (MSR == L1 && PAIR && !CSR && a.l1 && l1_plain(a)) return;  // k_assign_dense takes the pass
     if (a.n_dev) {  // launched for the largest count: tiles past the device count leave at once
         const uint64_t nd = *a.n_dev;
         if (row0 >= nd) return;
@@ -1248,6 +1249,52 @@ static int tiled_t(const AssignArgs &a, bool pair, bool big, cudaStream_t st, bo
     return MC_OK;
 }
 
+// smallest nonzero magnitude of v[0, m) and largest of the sums (0 where none is positive)
+__global__ void __launch_bounds__(256) k_l1_stat(const float *__restrict__ v, uint64_t m, const double *__restrict__ sums,
+                                                 uint64_t n, unsigned *vmin, unsigned long long *smax) {
+    unsigned mn = 0x7f800000u;
+    unsigned long long mx = 0ull;
+    const uint64_t i0 = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x, step = gridDim.x * uint64_t(blockDim.x);
+#pragma unroll 4
+    for (uint64_t i = i0; i < m; i += step) {
+        const unsigned b = __float_as_uint(v[i]) & 0x7fffffffu;
+        if (b) mn = min(mn, b);  // NaNs are above every finite magnitude
+    }
+    for (uint64_t i = i0; i < n; i += step) {
+        const double s = sums[i];
+        if (!(s <= 0.0)) {
+            const unsigned long long b = (unsigned long long)__double_as_longlong(s) & 0x7fffffffffffffffull;
+            mx = b > mx ? b : mx;
+        }
+    }
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) {
+        mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+        const unsigned long long y = __shfl_xor_sync(0xffffffffu, mx, o);
+        mx = y > mx ? y : mx;
+    }
+    if ((threadIdx.x & 31) == 0) {
+        atomicMin(vmin, mn);
+        atomicMax(smax, mx);
+    }
+}
+
+static int l1_stat(const float *v, uint64_t m, const double *sums, uint64_t n, unsigned *vmin, unsigned long long *smax,
+                   cudaStream_t st) {
+    MC_CUDA_TRY(cudaMemsetAsync(vmin, 0x7f, sizeof(unsigned), st));  // a NaN pattern: above every magnitude
+    MC_CUDA_TRY(cudaMemsetAsync(smax, 0, sizeof(unsigned long long), st));
+    k_l1_stat<<<unsigned(umin64((m + 1023) / 1024, 152 * 4)), 256, 0, st>>>(v, m, sums, n, vmin, smax), note_launch();
+    MC_CUDA_TRY(cudaGetLastError());
+    return MC_OK;
+}
+
+int launch_l1_row_stat(const float *X, uint64_t m, const double *rowsum, uint64_t n, L1Stat *stat, cudaStream_t st) {
+    return l1_stat(X, m, rowsum, n, &stat->xmin, &stat->xsum, st);
+}
+int launch_l1_center_stat(const float *C, uint64_t m, const double *csum, uint64_t k, L1Stat *stat, cudaStream_t st) {
+    return l1_stat(C, m, csum, k, &stat->cmin, &stat->csum, st);
+}
+
 uint32_t tiled_center_pad(uint32_t k, bool pair, int msr) {
     const uint32_t bn = pair ? 32 : ((msr == SQRL2 && k >= 128) ? 128 : 64);
     return (k + bn - 1) / bn * bn;
@@ -1257,6 +1304,10 @@ int launch_assign_tiled(const AssignArgs &a, bool csr, bool pair, cudaStream_t s
     if (a.n == 0) return MC_OK;
     // 8x8 register tiles for SQRL2 with many centers, 4x4 otherwise
     const bool big = (a.msr == SQRL2 && a.kp % 128 == 0);
+    if (!csr && pair && a.l1) {  // both are launched; one of them finds that the pass is the other's
+        bool done = false;
+        MC_TRY(launch_assign_dense(a, st, &done));
+    }
     if (!csr && !pair && !big) {
         bool done = false;
         MC_TRY(launch_assign_dense(a, st, &done));

@@ -4,6 +4,14 @@
 
 namespace mc {
 
+// What decides whether L1 with a pair-dependent prior equals plain L1 (l1_plain in
+// mc_assign_dev.cuh): the smallest nonzero magnitudes (float bits) and the largest sums (bits of
+// doubles, not below 0) of the rows and the centers.
+struct L1Stat {
+    unsigned long long xsum, csum;
+    unsigned xmin, cmin;
+};
+
 struct AssignArgs {
     int msr = SQRL2;
     uint64_t n = 0, d = 0;
@@ -34,6 +42,7 @@ struct AssignArgs {
     float *dmat = nullptr;
     uint64_t ldm = 0;
     int dmode = 0;
+    const L1Stat *l1 = nullptr;       // dense L1 in pair mode: set when the plain path may apply
 };
 
 __device__ __forceinline__ void write_dist(const AssignArgs &a, uint64_t row, uint32_t c, float v) {
@@ -67,6 +76,9 @@ constexpr uint64_t kL1UnionMaxEntries = 1ull << 29;
 // f(a, b) = a log a + b log b - (a + b) log((a + b) / 2) and a_cj the center transform
 int launch_jsd_ztable(const float *C, uint32_t k, uint64_t d, const double *csum, float pv, const float *gval,
                       uint32_t ngrp, double *ztab, cudaStream_t st);
+// row / center part of an L1Stat (dense rows; csum: the centers' sums)
+int launch_l1_row_stat(const float *X, uint64_t m, const double *rowsum, uint64_t n, L1Stat *stat, cudaStream_t st);
+int launch_l1_center_stat(const float *C, uint64_t m, const double *csum, uint64_t k, L1Stat *stat, cudaStream_t st);
 uint32_t tiled_center_pad(uint32_t k, bool pair, int msr);
 uint32_t sparse_center_pad(uint32_t k);
 

@@ -1,4 +1,4 @@
-// Exact FP32 assignment of dense rows with a constant prior (SQRL2, MKL): the
+// Exact FP32 assignment of dense rows (SQRL2, MKL with a constant prior, plain L1): the
 // argmin over centers of cmp::msr_with_prior (include/minicore/clustering/solve.h:234-285,
 // include/minicore/dist/applicator.h:1632-1915), columns sequential per (row, center), so it is
 // bit-identical to k_assign_tiled and the oracle's dense path.
@@ -33,6 +33,11 @@ __device__ __forceinline__ unsigned long long d2_sub(unsigned long long a, unsig
     asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
+__device__ __forceinline__ unsigned long long d2_add(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
 __device__ __forceinline__ unsigned long long d2_fma(unsigned long long a, unsigned long long b, unsigned long long c) {
     unsigned long long r;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
@@ -65,7 +70,8 @@ __device__ __forceinline__ void dense_step(const float *xs, int pitch, const flo
                         s = d2_fma(c0, d2_sub(c1, x[p]), s);
                     } else {
                         const unsigned long long df = d2_sub(c0, x[p]);
-                        s = d2_fma(df, df, s);
+                        if (MSR == L1) s = d2_add(s, df & 0x7fffffff7fffffffull);
+                        else s = d2_fma(df, df, s);
                     }
                 }
             }
@@ -128,7 +134,7 @@ struct DenseCta {
         else if (vec == 2) load_vec<2>(kb, cols);
         else load_vec<1>(kb, cols);
         __syncthreads();
-        if (MSR == SQRL2) return;
+        if (MSR == SQRL2 || MSR == L1) return;  // raw values
         // thread t: row t % BM (BM divides T or T divides BM)
         for (int r = t % BM; r < BM; r += T) {
             const uint64_t row = row0 + r;
@@ -249,6 +255,7 @@ template <int MSR, int WARPS>
 __global__ void __launch_bounds__(32 * WARPS, 12 / WARPS) k_assign_dense(const AssignArgs a, int kx, int vec) {
     extern __shared__ __align__(16) float dense_sm[];
     using Cta = DenseCta<MSR, WARPS>;
+    if (MSR == L1 && !l1_plain(a)) return;
     uint64_t nrows = a.n;
     if (a.n_dev) nrows = umin64(nrows, *a.n_dev);
     Cta cta{a, dense_sm, dense_sm + Cta::PITCH * kx, kx, vec, 0, nrows};
@@ -313,6 +320,8 @@ int launch_assign_dense(const AssignArgs &a, cudaStream_t st, bool *done) {
     const bool wide = a.n > 128 * 152 * 2;  // 128 rows per CTA, 64 where that leaves SMs without a tile
     if (a.msr == SQRL2) return wide ? dense_launch_w<SQRL2, 4>(a, st) : dense_launch_w<SQRL2, 2>(a, st);
     if (a.msr == MKL && a.k > 64) return wide ? dense_launch_w<MKL, 4>(a, st) : dense_launch_w<MKL, 2>(a, st);
+    // L1 in pair mode where its terms are plain differences (l1_plain): 100,000 x 64, k = 50: 105 -> 67 us (and 17 us for the CTAs that leave at once)
+    if (a.msr == L1 && a.l1) return wide ? dense_launch_w<L1, 4>(a, st) : dense_launch_w<L1, 2>(a, st);
     *done = false;
     return MC_OK;
 }

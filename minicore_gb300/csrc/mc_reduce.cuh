@@ -104,7 +104,7 @@ int launch_centroids(const CentroidArgs &a, SortWork &w, cudaStream_t st, bool p
 // nw_local > 0: the r-th row of a cluster (ascending) weighs weights[r], as the minibatch
 // update's weighted_median(rows(data, asp, nasn), ret, *weights) reads them (kmedian.h:335);
 // positions past nw_local take no part.
-int launch_l1_medians(const float *X, uint64_t d, uint32_t k, const SortWork &w, const double *weights,
+int launch_l1_medians(const float *X, uint64_t n, uint64_t d, uint32_t k, const SortWork &w, const double *weights,
                       float *centers, cudaStream_t st, uint64_t nw_local = 0);
 // the L1 restart's pass after reseeding center `id` at `center`: rows whose plain L1
 // distance (sequential float sum of |c - x|) is below their cost move to it
