@@ -126,6 +126,12 @@ int mc_uniforms(uint64_t seed, uint64_t offset, uint64_t m, double *out);
 int mc_kmeanspp(mc_context *ctx, const mc_matrix *X, uint32_t k, int msr, double prior,
                 const double *weights, const double *uniforms,
                 uint32_t *center_ids, uint32_t *asn, double *costs);
+/* mc_kmeanspp with the outputs in the types the reference's bindings return (python/smw.h:211-220,
+ * 329-341), converted on the device: asn as asn_bytes (1, 2 or 4) per row, costs as float32 where
+ * costs_f32 != 0, else double. */
+int mc_kmeanspp_narrow(mc_context *ctx, const mc_matrix *X, uint32_t k, int msr, double prior,
+                       const double *weights, const double *uniforms, uint32_t *center_ids, void *asn,
+                       int asn_bytes, void *costs, int costs_f32);
 /* Greedy k-means++ (n_local_trials > 1, kmeans.h:79-177; python/pydense.cpp:34-77): the
  * first center is the best of n_local_trials uniform picks; each later round draws
  * n_local_trials candidates from the distances without replacement and keeps the one with

@@ -271,6 +271,16 @@ def kmeanspp(matrix, k, *, msr=2, prior=0., seed=0, ntimes=1, lspp=0, expskips=0
     # CSR: the reference compares the extra runs against the first run's own cost
     # (python/smw.h:250), so the first run is always returned.
     runs = max(int(ntimes), 1) if M.kind == _lib.MC_DENSE_F32 else 1
+    if runs == 1 and not lspp and trials == 1:
+        # one run: assignments and costs come back in their final types, converted on the device
+        # (2M rows: 10 MB to copy instead of 24, and no pass over them here)
+        ids = np.empty(kk, dtype=np.uint32)
+        asn = np.empty(M.n, dtype=_asn_dtype(k))
+        costs = np.empty(M.n, dtype=np.float32 if M.kind == _lib.MC_DENSE_F32 else np.float64)
+        u = uniforms(seed, k)
+        check(_lib.load().mc_kmeanspp_narrow(ctx.handle, M.ref, k, _msr(msr), float(prior), _p(w), _p(u), _p(ids),
+                                             _p(asn), asn.itemsize, _p(costs), int(costs.dtype == np.float32)))
+        return ids, asn, costs
     best = None
     for t in range(runs):
         ids = np.empty(kk, dtype=np.uint32)

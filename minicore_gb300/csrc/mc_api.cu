@@ -2379,9 +2379,17 @@ int run_lspp(mc_context *ctx, const mc_matrix *X, const KmppArgs &a, uint32_t k,
 
 }  // namespace
 
+// asn as 1- or 2-byte integers (k at most 256 or 65536)
+template <class T>
+__global__ void k_narrow_asn(const uint32_t *__restrict__ a, uint64_t n, T *out) {
+    for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n; i += gridDim.x * uint64_t(blockDim.x))
+        out[i] = T(a[i]);
+}
+
+// asn: asn_bytes (1, 2 or 4) per row; costs: double, or float where costs_f32
 static int kmeanspp_impl(mc_context *ctx, const mc_matrix *X, uint32_t k, int msr, double prior, const double *weights,
                          const double *uniforms, uint32_t local_trials, uint64_t seed, uint32_t *center_ids,
-                         uint32_t *asn, double *costs, uint64_t lspp_rounds = 0) {
+                         void *asn, void *costs, uint64_t lspp_rounds = 0, int asn_bytes = 4, bool costs_f32 = false) {
     if (!ctx) return fail(MC_EINVAL, "ctx is null");
     if (!measure_supported(msr)) return fail(MC_EUNSUPPORTED, "measure not implemented on this path");
     if (!uniforms && local_trials <= 1) return fail(MC_EINVAL, "uniforms is null");
@@ -2449,8 +2457,25 @@ static int kmeanspp_impl(mc_context *ctx, const mc_matrix *X, uint32_t k, int ms
     else MC_TRY(run_kmeanspp(a, u.p, tmp.p, ctx->sms, st));
     if (lspp_rounds) MC_TRY(run_lspp(ctx, X, a, k, msr, prior, lspp_rounds, seed, ids.p, asnb.p, dist.p, tmp.p, st));
     MC_TRY(copy_out(center_ids, ids.p, k, st));
-    MC_TRY(copy_out(asn, asnb.p, n, st));
-    MC_TRY(copy_out(costs, dist.p, n, st));
+    DBuf<unsigned char> narrow;
+    DBuf<float> c32;
+    const unsigned og = unsigned(umin64((n + 255) / 256, uint64_t(ctx->sms) * 8));
+    if (asn && asn_bytes < 4) {
+        MC_TRY(narrow.alloc(n * uint64_t(asn_bytes), st));
+        if (asn_bytes == 1) k_narrow_asn<<<og, 256, 0, st>>>(asnb.p, n, narrow.p), note_launch();
+        else k_narrow_asn<<<og, 256, 0, st>>>(asnb.p, n, reinterpret_cast<uint16_t *>(narrow.p)), note_launch();
+        MC_TRY(copy_out(static_cast<unsigned char *>(asn), narrow.p, n * uint64_t(asn_bytes), st));
+    } else {
+        MC_TRY(copy_out(static_cast<uint32_t *>(asn), asnb.p, n, st));
+    }
+    if (costs && costs_f32) {
+        MC_TRY(c32.alloc(n, st));
+        k_costs_to_f32<<<og, 256, 0, st>>>(dist.p, n, c32.p), note_launch();
+        MC_TRY(copy_out(static_cast<float *>(costs), c32.p, n, st));
+    } else {
+        MC_TRY(copy_out(static_cast<double *>(costs), dist.p, n, st));
+    }
+    MC_CUDA_TRY(cudaGetLastError());
     MC_CUDA_TRY(cudaStreamSynchronize(st));
     return MC_OK;
 }
@@ -2460,6 +2485,15 @@ extern "C" {
 int mc_kmeanspp(mc_context *ctx, const mc_matrix *X, uint32_t k, int msr, double prior, const double *weights,
                 const double *uniforms, uint32_t *center_ids, uint32_t *asn, double *costs) {
     return kmeanspp_impl(ctx, X, k, msr, prior, weights, uniforms, 1, 0, center_ids, asn, costs);
+}
+
+int mc_kmeanspp_narrow(mc_context *ctx, const mc_matrix *X, uint32_t k, int msr, double prior, const double *weights,
+                       const double *uniforms, uint32_t *center_ids, void *asn, int asn_bytes, void *costs,
+                       int costs_f32) {
+    if (asn_bytes != 1 && asn_bytes != 2 && asn_bytes != 4) return fail(MC_EINVAL, "asn_bytes is 1, 2 or 4");
+    if (asn_bytes < 4 && k > (1u << (8 * asn_bytes))) return fail(MC_EINVAL, "asn_bytes too small for k");
+    return kmeanspp_impl(ctx, X, k, msr, prior, weights, uniforms, 1, 0, center_ids, asn, costs, 0, asn_bytes,
+                         costs_f32 != 0);
 }
 
 int mc_kmeanspp_ex(mc_context *ctx, const mc_matrix *X, uint32_t k, int msr, double prior, const double *weights,
