@@ -270,7 +270,11 @@ struct mc_job {
     DBuf<uint32_t> grp;
     DBuf<float> gval;
     DBuf<double> ztab;
+    DBuf<float> jlogs;      // centers' a and a log a
     uint32_t ngrp = 0;
+    // rows listed by group, for k_assign_jsd_groups (jgroups: it takes this job's passes)
+    bool jgroups = false;
+    JsdGroupWork jgw;
     SortWork sort;
     L1CsrWork l1csr;  // L1 medians over CSR rows
     DBuf<L1Stat> l1stat;  // dense L1 in pair mode: the rows' part is written at creation
@@ -415,12 +419,23 @@ int job_assign_with(mc_job *j, const float *C, double prior_sum, bool force_exac
     }
     if (sparse && j->msr == JSD) {
         MC_TRY(j->ztab.alloc(uint64_t(j->ngrp) * j->k, j->st));
-        MC_TRY(launch_jsd_ztable(C, j->k, d, j->csum.p, j->pv, j->gval.p, j->ngrp, j->ztab.p, j->st));
+        MC_TRY(j->jlogs.alloc(2 * uint64_t(jsd_log_centers(j->k, d)) * d, j->st));
+        MC_TRY(launch_jsd_ztable(C, j->k, d, j->csum.p, j->pv, j->gval.p, j->ngrp, j->ztab.p, j->jlogs.p, j->st));
         a.grp = j->grp.p;
         a.ztab = j->ztab.p;
     }
     if (sparse) {
         Phase ph("assign_csr_sparse", j->st);
+        if (j->jgroups) {
+            JsdGroups g;
+            g.nbucket = j->ngrp + 1;
+            g.perm = j->jgw.sort.perm.p;
+            g.start = j->jgw.sort.bucket_start.p;
+            g.count = j->jgw.sort.bucket_count.p;
+            g.slab_start = j->jgw.slabs.p;
+            g.bx = j->jgw.bx.p;
+            return launch_assign_jsd_groups(a, g, j->st);
+        }
         return launch_assign_sparse(a, j->st, j->ctx->sms);
     }
     Phase ph(csr ? "assign_csr_tiled" : "assign_dense_fp32", j->st);
@@ -1541,6 +1556,12 @@ static int job_create_impl(mc_context *ctx, const mc_matrix *X, const float *cen
         MC_TRY(launch_l1_row_stat(j->M.X, n * d, j->rowsum.p, n, j->l1stat.p, st));
     }
     j->sparse_path = j->M.kind == MC_CSR_F32 && !j->pair && (msr != JSD || j->ngrp > 0);
+    if (j->sparse_path && msr == JSD && jsd_groups_pay(n, d, k, j->M.nnz, j->ngrp)) {
+        MC_TRY(jsd_bucket_rows(j->grp.p, n, j->ngrp, j->M.nnz, d, ctx->sms, j->jgw, st));
+        MC_TRY(j->jgw.bx.alloc(n, st));
+        MC_TRY(launch_jsd_row_terms(j->M.vals, j->M.indptr, n, j->rsi.p, j->rinc.p, j->jgw.bx.p, ctx->sms, st));
+        j->jgroups = true;
+    }
     *out = j.release();
     return MC_OK;
 }

@@ -73,12 +73,32 @@ uint64_t l1_union_work_entries(uint32_t k, uint64_t d);
 // the largest work space (in entries) for which the union kernel is used
 constexpr uint64_t kL1UnionMaxEntries = 1ull << 29;
 // JSD sparse-dot table: ztab[g * k + c] = sum over all columns j of f(a_cj, gval[g]) with
-// f(a, b) = a log a + b log b - (a + b) log((a + b) / 2) and a_cj the center transform
+// f(a, b) = a log a + b log b - (a + b) log((a + b) / 2) and a_cj the center transform; alog: 2 d
+// jsd_log_centers() floats of work space (the transform and a log a of that many centers at a time)
+uint32_t jsd_log_centers(uint32_t k, uint64_t d);
 int launch_jsd_ztable(const float *C, uint32_t k, uint64_t d, const double *csum, float pv, const float *gval,
-                      uint32_t ngrp, double *ztab, cudaStream_t st);
+                      uint32_t ngrp, double *ztab, float *alog, cudaStream_t st);
 // row / center part of an L1Stat (dense rows; csum: the centers' sums)
 int launch_l1_row_stat(const float *X, uint64_t m, const double *rowsum, uint64_t n, L1Stat *stat, cudaStream_t st);
 int launch_l1_center_stat(const float *C, uint64_t m, const double *csum, uint64_t k, L1Stat *stat, cudaStream_t st);
+// JSD over CSR rows grouped by their zero-entry value (mc_assign_jsd.cu): bucket 0 holds the
+// rows of groups too small for a table, the others one group each, largest first
+struct JsdGroups {
+    uint32_t nbucket = 0;
+    const uint32_t *perm = nullptr;                     // [n] rows by bucket
+    const uint64_t *start = nullptr, *count = nullptr;  // [nbucket] of perm
+    const uint64_t *slab_start = nullptr;               // [nbucket + 1] slabs of rows before each bucket
+    const double *bx = nullptr;                         // [n] row terms
+};
+struct JsdGroupWork;
+// whether k_assign_jsd_groups takes a job's passes
+bool jsd_groups_pay(uint64_t n, uint64_t d, uint32_t k, uint64_t nnz, uint32_t ngrp);
+int launch_jsd_row_terms(const float *vals, const uint64_t *indptr, uint64_t n, const float *rsi, const float *rinc,
+                         double *bx, int sms, cudaStream_t st);
+// rows listed by bucket into w
+int jsd_bucket_rows(const uint32_t *grp, uint64_t n, uint32_t ngrp, uint64_t nnz, uint64_t d, int sms, JsdGroupWork &w,
+                    cudaStream_t st);
+int launch_assign_jsd_groups(const AssignArgs &a, const JsdGroups &jg, cudaStream_t st);
 uint32_t tiled_center_pad(uint32_t k, bool pair, int msr);
 uint32_t sparse_center_pad(uint32_t k);
 

@@ -715,6 +715,12 @@ static uint64_t sort_tile_rows(uint64_t n, uint32_t k) {
     return n <= (1u << 19) && uint64_t(k) * (n / 512) <= (1u << 19) ? 512 : kSortTile;
 }
 
+int launch_scan_ceil_div(const uint64_t *in, uint64_t *out, uint64_t m, uint64_t div, cudaStream_t st) {
+    k_exclusive_scan_u64<<<1, 1024, 0, st>>>(in, out, m, div), note_launch();
+    MC_CUDA_TRY(cudaGetLastError());
+    return MC_OK;
+}
+
 int launch_sort_by_key(const uint32_t *keys, const uint32_t *keys2, uint64_t n, uint32_t k, SortWork &w,
                        cudaStream_t st) {
     const uint64_t tile_rows = sort_tile_rows(n, k);

@@ -19,6 +19,12 @@ struct SortWork {
     bool bands_ready = false;     // bands holds the offsets of the owning job's matrix
 };
 
+struct JsdGroupWork {  // rows of a CSR JSD job by bucket
+    SortWork sort;
+    DBuf<uint64_t> slabs;  // [buckets + 1]
+    DBuf<double> bx;       // [n] row terms
+};
+
 struct CentroidArgs {
     bool csr = false;
     uint64_t n = 0, d = 0;
@@ -135,6 +141,8 @@ int launch_l1_reseed_update_csr(const float *vals, const uint32_t *idx, const ui
 // scratch: optional work space (kept by the caller, so that a captured graph allocates nothing)
 int launch_exclusive_scan_u64(const uint64_t *in, uint64_t *out, uint64_t m, cudaStream_t st,
                               DBuf<uint64_t> *scratch = nullptr);
+// out[i] = sum over q < i of ceil(in[q] / div), out[m] the total (one CTA)
+int launch_scan_ceil_div(const uint64_t *in, uint64_t *out, uint64_t m, uint64_t div, cudaStream_t st);
 int launch_center_sums(const float *C, uint32_t k, uint64_t d, double *csum, float *cnorm, cudaStream_t st);
 
 }  // namespace mc
