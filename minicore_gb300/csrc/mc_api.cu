@@ -363,9 +363,10 @@ struct DistOut {
 int job_assign_with(mc_job *j, const float *C, double prior_sum, bool force_exact, const DistOut *dout = nullptr,
                     bool graph_mode = false) {
     const uint64_t n = j->M.n, d = j->M.d;
-    MC_TRY(launch_center_sums(C, j->k, d, j->csum.p, j->cnorm.p, j->st));
     const bool csr = j->M.kind == MC_CSR_F32;
     const bool tc = !csr && !force_exact && !dout && j->msr == SQRL2 && j->precision != MC_FP32;
+    // the norms, a sequential chain over the columns, serve the tensor-core pass only
+    MC_TRY(launch_center_sums(C, j->k, d, j->csum.p, tc ? j->cnorm.p : nullptr, j->st));
     if (tc) {
         MC_TRY(tc_assign(j->tc, j->M.X, n, d, C, j->cnorm.p, j->k, j->precision, j->rownorm.p, j->asn.p,
                          j->costs.p, j->ctx->sms, j->st, &j->last_recheck, graph_mode));
@@ -1532,7 +1533,7 @@ static int job_create_impl(mc_context *ctx, const mc_matrix *X, const float *cen
     // constant-prior check: pv == prior for every pair when prior >= smallest_pv at the
     // largest row and center sums (centers are means or rows, so bounded by the rows)
     if (msr != SQRL2) {
-        MC_TRY(launch_center_sums(j->C.p, k, d, j->csum.p, j->cnorm.p, st));
+        MC_TRY(launch_center_sums(j->C.p, k, d, j->csum.p, nullptr, st));
         std::vector<double> rs(n), cs(k);
         MC_CUDA_TRY(cudaMemcpyAsync(rs.data(), j->rowsum.p, n * sizeof(double), cudaMemcpyDeviceToHost, st));
         MC_CUDA_TRY(cudaMemcpyAsync(cs.data(), j->csum.p, k * sizeof(double), cudaMemcpyDeviceToHost, st));

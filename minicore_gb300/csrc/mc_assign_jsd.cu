@@ -6,13 +6,14 @@
 // m1 = a_cj + b.  The m0 half depends on (group, column, center) only: where a group's rows have
 // more entries than there are columns it is tabulated once per CTA instead of once per entry, which
 // halves the logarithms, and they bound this pass: 50,000 rows of 1500 entries, 850 groups, 20,000
-// columns, k = 50: 8.2 ms in k_assign_sparse, 7.1 here, instruction issue 88 % busy.  A CTA takes up to 96 rows of one group and walks
-// the columns in bands of kJsdBand through shared memory: the center transform (double buffered by
-// cp.async) and the band's table.  Rows of groups too small for a table share CTAs without one.  A
-// warp visits its rows in turn in each band (sums and cursors wait in shared memory, so one copy of
-// the code serves all rows: unrolled over eight rows in registers it ran out of the instruction
-// cache: 97 ms), lane = two centers, the row's next 32 entries one per lane.  Per (row, center) the
-// terms and their order are those of k_assign_sparse, so the results are bit-identical to it.
+// columns, k = 50: 8.2 ms in k_assign_sparse, 7.1 here, instruction issue 88 % busy.  A CTA takes up
+// to 96 rows of one group and walks the columns in bands of kJsdBand through shared memory: the
+// center transform (double buffered by cp.async) and the band's table.  Rows of groups too small for
+// a table share CTAs without one.  A warp visits its rows in turn in each band (sums and cursors
+// wait in shared memory, so one copy of the code serves all rows: unrolled over eight rows in
+// registers it ran out of the instruction cache: 97 ms), lane = two centers, the row's next 32
+// entries one per lane.  Per (row, center) the terms and their order are those of k_assign_sparse,
+// so the results are bit-identical to it.
 #include "mc_assign_dev.cuh"
 #include "mc_reduce.cuh"
 

@@ -1176,37 +1176,46 @@ int launch_centroids(const CentroidArgs &a, SortWork &w, cudaStream_t st, bool p
 // ------------------------------------------------------------------------------------
 // per-center sums (sequential FP64 over columns) and squared norms
 // ------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) k_center_sums(const float *__restrict__ C, uint32_t k, uint64_t d, double *csum,
+__global__ void __launch_bounds__(32) k_center_sums(const float *__restrict__ C, uint32_t k, uint64_t d, double *csum,
                                                      float *cnorm) {
-    // one warp per center.  csum: lane l adds columns l, l+32, l+64, ... in FP64, then the 32
+    // one warp, a CTA of its own, per center: the FP64 chain of a lane bounds it (20,000 columns: 625
+    // adds of 75 ns), and warps that share an SM share its FP64 pipe (k = 50: 142 us with the norms
+    // and four warps per CTA, 61 without).  csum: lane l adds columns l, l+32, l+64, ... in FP64, then the 32
     // lane partials are added in lane order (the canonical center-sum order).  cnorm: a FP32
     // fmaf chain in column order, by lane 0 from coalesced shared-memory chunks.
-    __shared__ float t[4][256];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const uint32_t c = blockIdx.x * 4 + w;
-    if (c >= k) return;  // whole warp; the block has no barrier
+    __shared__ float t[256];
+    const int lane = threadIdx.x;
+    const uint32_t c = blockIdx.x;
     const float *r = C + uint64_t(c) * d;
     double s = 0.0;
     float q = 0.f;
+    // the next 256 columns are on their way while these are added
+    float x[8], y[8];
+    auto load = [&](uint64_t j0, float (&v)[8]) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = j0 + lane + 32 * u < d ? r[j0 + lane + 32 * u] : 0.f;
+    };
+    load(0, x);
     for (uint64_t j0 = 0; j0 < d; j0 += 256) {
         const int cnt = int(d - j0 < 256 ? d - j0 : 256);
+        load(j0 + 256, y);
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
             const int i = lane + 32 * u;
             if (i < cnt) {
-                const float x = r[j0 + i];
-                s = s + double(x);
-                if (cnorm) t[w][i] = x;
+                s = s + double(x[u]);
+                if (cnorm) t[i] = x[u];
             }
+            x[u] = y[u];
         }
         if (cnorm) {
             __syncwarp();
             if (lane == 0) {
                 if (cnt == 256) {
 #pragma unroll 16
-                    for (int i = 0; i < 256; ++i) q = fmaf(t[w][i], t[w][i], q);
+                    for (int i = 0; i < 256; ++i) q = fmaf(t[i], t[i], q);
                 } else {
-                    for (int i = 0; i < cnt; ++i) q = fmaf(t[w][i], t[w][i], q);
+                    for (int i = 0; i < cnt; ++i) q = fmaf(t[i], t[i], q);
                 }
             }
             __syncwarp();
@@ -1223,7 +1232,7 @@ __global__ void __launch_bounds__(128) k_center_sums(const float *__restrict__ C
 
 int launch_center_sums(const float *C, uint32_t k, uint64_t d, double *csum, float *cnorm, cudaStream_t st) {
     if (k == 0) return MC_OK;
-    k_center_sums<<<(k + 3) / 4, 128, 0, st>>>(C, k, d, csum, cnorm), note_launch();
+    k_center_sums<<<k, 32, 0, st>>>(C, k, d, csum, cnorm), note_launch();
     MC_CUDA_TRY(cudaGetLastError());
     return MC_OK;
 }
