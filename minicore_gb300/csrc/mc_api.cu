@@ -1556,6 +1556,7 @@ static int job_create_impl(mc_context *ctx, const mc_matrix *X, const float *cen
         MC_TRY(j->l1stat.alloc(1, st));
         MC_TRY(launch_l1_row_stat(j->M.X, n * d, j->rowsum.p, n, j->l1stat.p, st));
     }
+    j->sort.chunk_rows = centroid_chunk_rows(j->M.kind == MC_CSR_F32);
     j->sparse_path = j->M.kind == MC_CSR_F32 && !j->pair && (msr != JSD || j->ngrp > 0);
     if (j->sparse_path && msr == JSD && jsd_groups_pay(n, d, k, j->M.nnz, j->ngrp)) {
         MC_TRY(jsd_bucket_rows(j->grp.p, n, j->ngrp, j->M.nnz, d, ctx->sms, j->jgw, st));

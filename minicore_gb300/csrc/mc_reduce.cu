@@ -505,10 +505,14 @@ __global__ void k_sort_count(const uint32_t *__restrict__ keys, const uint32_t *
 }
 
 // one CTA per key: exclusive scan of the key's tile counts (in place: per-tile offsets
-// relative to the bucket start) and the bucket total
+// relative to the bucket start) and the bucket total.  The last CTA to finish (ticket, which it
+// resets) also scans the totals into bucket_start and, with ch > 0, their chunks of ch rows into
+// chunk_start: in launches of their own the two scans took 2.6 us each, all latency.
 __global__ void __launch_bounds__(256) k_sort_key_scan(uint32_t *tile_counts, uint64_t ntiles, uint32_t k,
-                                                       uint64_t *bucket_count) {
-    __shared__ uint64_t wsum[8];
+                                                       uint64_t *bucket_count, unsigned *ticket,
+                                                       uint64_t *bucket_start, uint64_t ch, uint64_t *chunk_start) {
+    __shared__ uint64_t wsum[8], wsum2[8];
+    __shared__ bool last;
     const uint32_t key = blockIdx.x;
     if (key >= k) return;
     uint32_t *row = tile_counts + uint64_t(key) * ntiles;
@@ -529,12 +533,54 @@ __global__ void __launch_bounds__(256) k_sort_key_scan(uint32_t *tile_counts, ui
     uint64_t wbase = 0;
     for (int i = 0; i < w; ++i) wbase += wsum[i];
     uint64_t acc = wbase + incl - s;
+    if (t == 255) {
+        bucket_count[key] = acc + s;
+        if (ticket) {
+            __threadfence();
+            last = atomicAdd(ticket, 1u) == k - 1;
+        }
+    }
     for (uint64_t i = b; i < e; ++i) {
         const uint32_t c = row[i];
         row[i] = uint32_t(acc);
         acc += c;
     }
-    if (t == 255) bucket_count[key] = acc;
+    if (!ticket) return;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    if (t == 0) *ticket = 0;
+    // thread t: the keys [t q, t q + q)
+    const uint32_t q = (k + 255) / 256, k0 = umin64(k, uint64_t(t) * q), k1 = umin64(k, uint64_t(k0) + q);
+    uint64_t s1 = 0, s2 = 0;
+    for (uint32_t i = k0; i < k1; ++i) {
+        const uint64_t v = __ldcg(bucket_count + i);
+        s1 += v;
+        if (ch) s2 += (v + ch - 1) / ch;
+    }
+    uint64_t i1 = s1, i2 = s2;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const uint64_t v1 = __shfl_up_sync(0xffffffffu, i1, off), v2 = __shfl_up_sync(0xffffffffu, i2, off);
+        if (lane >= off) i1 += v1, i2 += v2;
+    }
+    if (lane == 31) wsum[w] = i1, wsum2[w] = i2;
+    __syncthreads();
+    uint64_t a1 = i1 - s1, a2 = i2 - s2;
+    for (int i = 0; i < w; ++i) a1 += wsum[i], a2 += wsum2[i];
+    for (uint32_t i = k0; i < k1; ++i) {
+        const uint64_t v = __ldcg(bucket_count + i);
+        bucket_start[i] = a1;
+        a1 += v;
+        if (ch) {
+            chunk_start[i] = a2;
+            a2 += (v + ch - 1) / ch;
+        }
+    }
+    if (t == 255) {
+        bucket_start[k] = a1;
+        if (ch) chunk_start[k] = a2;
+    }
 }
 
 // exclusive scan of up to a few thousand counts (single CTA of 1024 threads): per-thread
@@ -708,6 +754,8 @@ int launch_exclusive_scan_u64(const uint64_t *in, uint64_t *out, uint64_t m, cud
     return MC_OK;
 }
 
+constexpr uint32_t kFusedScanKeys = 4096;
+
 // Rows per sort tile (any size gives the same permutation).  A tile's rows are scattered by one
 // warp, 32 after 32, so short tiles finish sooner (10,000 rows: 15.4 -> 5 us with 512 rows); every
 // tile costs k counts, written, scanned and read, so long lists and many keys keep 2048.
@@ -734,8 +782,23 @@ int launch_sort_by_key(const uint32_t *keys, const uint32_t *keys2, uint64_t n, 
         k_sort_count<<<unsigned(ntiles), 256, 0, st>>>(keys, keys2, n, k, ntiles, tile_rows, w.tile_counts.p), note_launch();
     else
         MC_CUDA_TRY(cudaMemsetAsync(w.bucket_count.p, 0, k * sizeof(uint64_t), st));
-    if (ntiles) k_sort_key_scan<<<k, 256, 0, st>>>(w.tile_counts.p, ntiles, k, w.bucket_count.p), note_launch();
-    k_exclusive_scan_u64<<<1, 1024, 0, st>>>(w.bucket_count.p, w.bucket_start.p, k, 0), note_launch();
+    // past a few thousand keys the last CTA's 256 threads would scan too many each
+    const bool fused = ntiles && k <= kFusedScanKeys;
+    w.chunk_done = 0;
+    if (fused) {
+        if (!w.ticket.p) {
+            MC_TRY(w.ticket.alloc(1, st));
+            MC_CUDA_TRY(cudaMemsetAsync(w.ticket.p, 0, sizeof(unsigned), st));
+        }
+        if (w.chunk_rows) MC_TRY(w.chunk_start.alloc(uint64_t(k) + 1, st));
+        w.chunk_done = w.chunk_rows;
+    }
+    if (ntiles)
+        k_sort_key_scan<<<k, 256, 0, st>>>(w.tile_counts.p, ntiles, k, w.bucket_count.p, fused ? w.ticket.p : nullptr,
+                                           w.bucket_start.p, w.chunk_rows, w.chunk_start.p),
+            note_launch();
+    if (!fused)
+        k_exclusive_scan_u64<<<1, 1024, 0, st>>>(w.bucket_count.p, w.bucket_start.p, k, 0), note_launch();
     if (ntiles) {
         if (!keys2)
             k_sort_scatter<<<unsigned(ntiles), 32, k <= kSmemKeys ? k * sizeof(uint32_t) : 0, st>>>(
@@ -764,6 +827,8 @@ int launch_sort_by_key(const uint32_t *keys, const uint32_t *keys2, uint64_t n, 
 // 319 us (300 at the copy rate); 300,001 x 100, k = 200: 47 -> 28; 10,000 x 50, k = 25: 19.8 -> 11.5
 // (the round trips of 256 dependent rows).  Before: a thread per column, batches of eight.
 constexpr uint64_t kDenseChunk = 256;
+
+uint64_t centroid_chunk_rows(bool csr) { return csr ? 4096 : kDenseChunk; }
 
 template <int V>
 struct ColVec;
@@ -1129,11 +1194,16 @@ __global__ void k_centroid_singletons_csr(const float *__restrict__ vals, const 
 int launch_centroids(const CentroidArgs &a, SortWork &w, cudaStream_t st, bool presorted) {
     const uint64_t n = a.n, d = a.d;
     const uint32_t k = a.k;
-    const uint64_t ch = a.csr ? 4096 : kDenseChunk;
-    if (!presorted) MC_TRY(launch_sort_by_key(a.keys, a.keys2, n, k, w, st));
-    MC_TRY(w.chunk_start.alloc(uint64_t(k) + 1, st));
-    // chunk starts: exclusive scan of ceil(bucket count / ch)
-    k_exclusive_scan_u64<<<1, 1024, 0, st>>>(w.bucket_count.p, w.chunk_start.p, k, ch), note_launch();
+    const uint64_t ch = centroid_chunk_rows(a.csr);
+    if (!presorted) {
+        w.chunk_rows = ch;
+        MC_TRY(launch_sort_by_key(a.keys, a.keys2, n, k, w, st));
+    }
+    // chunk starts: exclusive scan of ceil(bucket count / ch), unless the sort wrote them
+    if (w.chunk_done != ch) {
+        MC_TRY(w.chunk_start.alloc(uint64_t(k) + 1, st));
+        k_exclusive_scan_u64<<<1, 1024, 0, st>>>(w.bucket_count.p, w.chunk_start.p, k, ch), note_launch();
+    }
     const uint64_t members = n + (a.keys2 ? a.extra_members : 0);
     const uint64_t max_chunks = (members + ch - 1) / ch + k;
     MC_TRY(w.partial.alloc(max_chunks * d, st));

@@ -16,6 +16,9 @@ struct SortWork {
     DBuf<double> partial;         // [chunks][d]
     DBuf<double> partial_w;       // [chunks]
     DBuf<uint32_t> bands;         // CSR centroid sums: [n][bands + 1] row offsets of the column bands
+    DBuf<unsigned> ticket;        // k_sort_key_scan's, zero between sorts
+    uint64_t chunk_rows = 0;      // > 0: a sort also writes chunk_start for chunks of this many rows
+    uint64_t chunk_done = 0;      // the chunk rows that chunk_start was last written for by a sort
     bool bands_ready = false;     // bands holds the offsets of the owning job's matrix
 };
 
@@ -100,6 +103,7 @@ int launch_sort_by_key(const uint32_t *keys, const uint32_t *keys2, uint64_t n, 
 int launch_centroid_chunks_csr(const CentroidArgs &a, SortWork &w, uint64_t max_chunks, uint64_t ch, cudaStream_t st,
                                bool *done);
 // presorted: w already holds the counting sort of a.keys (no second membership)
+uint64_t centroid_chunk_rows(bool csr);  // rows per chunk of the centroid sums
 int launch_centroids(const CentroidArgs &a, SortWork &w, cudaStream_t st, bool presorted = false);
 
 // L1 centers over dense rows (set_centroids_l1, clustering/centroid.h:435-504), from the
