@@ -324,7 +324,7 @@ int mc_server_destroy(mc_server *s);
 
 /* Kernel-variant autotuner (no reference counterpart).  Some kernels come in variants that
  * compute bit-identical results (same per-element arithmetic and summation order) at
- * different speeds: the CSR sparse-dot batch size, the SQRL2 FP32 register tile and the
+ * different speeds: the CSR sparse-dot batch size, the SQRL2 FP32 kernel and the
  * kmeans++ distance-update load path.  The first call for a shape bucket times each variant
  * and keeps the fastest.  Decisions persist in a cache file (MC_AUTOTUNE_CACHE, default
  * $XDG_CACHE_HOME or $HOME/.cache + /minicore_gb300/autotune.tsv); MC_AUTOTUNE=0 or

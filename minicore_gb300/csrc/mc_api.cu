@@ -1559,10 +1559,13 @@ static int job_create_impl(mc_context *ctx, const mc_matrix *X, const float *cen
     j->sort.chunk_rows = centroid_chunk_rows(j->M.kind == MC_CSR_F32);
     j->sparse_path = j->M.kind == MC_CSR_F32 && !j->pair && (msr != JSD || j->ngrp > 0);
     if (j->sparse_path && msr == JSD && jsd_groups_pay(n, d, k, j->M.nnz, j->ngrp)) {
-        MC_TRY(jsd_bucket_rows(j->grp.p, n, j->ngrp, j->M.nnz, d, ctx->sms, j->jgw, st));
-        MC_TRY(j->jgw.bx.alloc(n, st));
-        MC_TRY(launch_jsd_row_terms(j->M.vals, j->M.indptr, n, j->rsi.p, j->rinc.p, j->jgw.bx.p, ctx->sms, st));
-        j->jgroups = true;
+        int rc = jsd_bucket_rows(j->grp.p, n, j->ngrp, j->M.nnz, d, ctx->sms, j->jgw, st);
+        if (rc == MC_OK) rc = j->jgw.bx.alloc(n, st);
+        if (rc == MC_OK)
+            rc = launch_jsd_row_terms(j->M.vals, j->M.indptr, n, j->rsi.p, j->rinc.p, j->jgw.bx.p, ctx->sms, st);
+        if (rc != MC_OK && rc != MC_ENOMEM) return rc;
+        if (rc == MC_ENOMEM) cudaGetLastError();  // no room for the lists: the gather kernels
+        j->jgroups = rc == MC_OK;
     }
     *out = j.release();
     return MC_OK;

@@ -365,7 +365,8 @@ static int band_launch(const CentroidArgs &a, SortWork &w, uint64_t max_chunks, 
     return MC_OK;
 }
 
-// *done = false: neither kernel applies (very wide and sparse rows: k_centroid_chunks_csr)
+// *done = false: neither kernel applies (very wide and sparse rows, or no memory for the band
+// offsets: k_centroid_chunks_csr)
 int launch_centroid_chunks_csr(const CentroidArgs &a, SortWork &w, uint64_t max_chunks, uint64_t ch, cudaStream_t st,
                                bool *done) {
     const uint64_t n = a.n, d = a.d;
@@ -383,7 +384,11 @@ int launch_centroid_chunks_csr(const CentroidArgs &a, SortWork &w, uint64_t max_
     if (shift) {
         const uint32_t nb = uint32_t((d + (uint64_t(1) << shift) - 1) >> shift);
         if (!a.keep_bands || !w.bands_ready) {
-            MC_TRY(w.bands.alloc(n * (uint64_t(nb) + 1), st));
+            if (w.bands.alloc(n * (uint64_t(nb) + 1), st) != MC_OK) {  // no room for the offsets
+                cudaGetLastError();
+                *done = false;
+                return MC_OK;
+            }
             k_csr_band_offsets<<<unsigned(umin64((n + 7) / 8, 152 * 8)), 256, 0, st>>>(a.idx, a.indptr, n, shift, nb,
                                                                                      w.bands.p), note_launch();
             MC_CUDA_TRY(cudaGetLastError());
