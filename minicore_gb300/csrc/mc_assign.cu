@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(256) k_assign_tiled(AssignArgs a) {
     __shared__ uint64_t cursor[CSR ? BM : 1];
 
     const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
-    const uint64_t row0 = uint64_t(blockIdx.x) * BM;
+    uint64_t row0 = uint64_t(blockIdx.x) * BM;
     const uint64_t d = a.d;
     if (MSR == L1 && PAIR && !CSR && a.l1 && l1_plain(a)) return;  // k_assign_dense takes the pass
     if (a.n_dev) {  // launched for the largest count: tiles past the device count leave at once
@@ -267,6 +267,10 @@ __global__ void __launch_bounds__(256) k_assign_tiled(AssignArgs a) {
         if (nd < a.n) a.n = nd;
     }
 
+    // L1 pairs over dense rows: a resident grid strides over the tiles, so that a pass that is
+    // k_assign_dense's costs two CTAs per SM that leave at once, not one per tile (17 -> 4 us, 100,000 rows)
+    constexpr bool kStride = MSR == L1 && PAIR && !CSR;
+    do {
     float rpv = a.pv;
     Best best[TM];
 #pragma unroll
@@ -441,6 +445,8 @@ __global__ void __launch_bounds__(256) k_assign_tiled(AssignArgs a) {
             }
         }
     }
+    row0 += uint64_t(gridDim.x) * BM;
+    } while (kStride && row0 < a.n);
 }
 
 // ------------------------------------------------------------------------------------
@@ -1274,7 +1280,10 @@ template <int MSR, bool CSR>
 static int tiled_t(const AssignArgs &a, bool pair, bool big, cudaStream_t st, bool tune) {
     if (pair) {
         constexpr int BM = 32;
-        k_assign_tiled<MSR, true, 2, 2, CSR><<<unsigned((a.n + BM - 1) / BM), 256, 0, st>>>(a), note_launch();
+        const uint64_t tiles = (a.n + BM - 1) / BM;
+        const bool stride = MSR == L1 && !CSR && a.l1;
+        k_assign_tiled<MSR, true, 2, 2, CSR><<<unsigned(stride ? umin64(tiles, 152 * 2) : tiles), 256, 0, st>>>(a),
+            note_launch();
     } else if (big) {
         // SQRL2 with kp % 128 == 0: 8x8 register tiles (128 rows per CTA) or 4x4 (64 rows), dense
         // rows k_assign_dense or 8x8; same per-pair arithmetic, so the autotuner may pick either
