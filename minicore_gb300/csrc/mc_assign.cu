@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(256) k_assign_tiled(AssignArgs a) {
     if (MSR == L1 && PAIR && !CSR && a.l1 && l1_plain(a)) return;  // k_assign_dense takes the pass
     if (a.n_dev) {  // launched for the largest count: tiles past the device count leave at once
         const uint64_t nd = *a.n_dev;
-        if (row0 >= nd) return;
+        if (row0 >= nd || assign_few_takes(a, nd)) return;
         if (nd < a.n) a.n = nd;
     }
 
@@ -1360,8 +1360,73 @@ uint32_t tiled_center_pad(uint32_t k, bool pair, int msr) {
     return (k + bn - 1) / bn * bn;
 }
 
+// SQRL2 over a short list of rows (the tensor-core path's rescans): four rows per CTA, a center per
+// thread, columns in order.  A tile kernel puts such a list on a few SMs and takes a whole tile's
+// time for it: 60,000 x 128, k = 40, a Lloyd update's list: 23.5 us, here 14.0.
+__global__ void __launch_bounds__(128) k_assign_few(const AssignArgs a) {
+    extern __shared__ float4 few_x[];  // [d], the four rows' values of a column
+    __shared__ Best wb[4][4];
+    const uint64_t nd = a.n_dev ? umin64(a.n, *a.n_dev) : a.n;
+    if (!assign_few_takes(a, nd)) return;
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const uint32_t d = uint32_t(a.d);
+    float *xf = reinterpret_cast<float *>(few_x);
+    for (uint64_t r0 = uint64_t(blockIdx.x) * 4; r0 < nd; r0 += uint64_t(gridDim.x) * 4) {
+        __syncthreads();  // the rows and bests of the four before are read
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const bool live = r0 + r < nd;
+            const float *src = a.X + uint64_t(live ? a.rows[r0 + r] : a.rows[r0]) * d;
+            for (uint32_t j = t; j < d; j += 128) xf[4 * j + r] = src[j];
+        }
+        __syncthreads();
+        Best b[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) best_init(b[r]);
+        for (uint32_t c = t; c < a.k; c += 128) {
+            float acc[4] = {0.f, 0.f, 0.f, 0.f};
+            const float *ct = a.CT0 + c;
+#pragma unroll 16
+            for (uint32_t j = 0; j < d; ++j) {
+                const float cv = __ldg(ct + uint64_t(j) * a.kp);
+                const float4 x = few_x[j];
+                const float d0 = cv - x.x, d1 = cv - x.y, d2 = cv - x.z, d3 = cv - x.w;
+                acc[0] = fmaf(d0, d0, acc[0]);
+                acc[1] = fmaf(d1, d1, acc[1]);
+                acc[2] = fmaf(d2, d2, acc[2]);
+                acc[3] = fmaf(d3, d3, acc[3]);
+            }
+#pragma unroll
+            for (int r = 0; r < 4; ++r) best_offer(b[r], finish_key<SQRL2>(acc[r]), c);
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+#pragma unroll
+            for (int m = 16; m >= 1; m >>= 1) best_merge_shfl(b[r], m);
+            if (lane == 0) wb[r][w] = b[r];
+        }
+        __syncthreads();
+        if (t < 4 && r0 + t < nd) {
+            Best v = wb[t][0];
+            for (int i = 1; i < 4; ++i)
+                if (wb[t][i].v < v.v || (wb[t][i].v == v.v && wb[t][i].j < v.j)) v = wb[t][i];
+            const bool nan0 = v.v == __int_as_float(0xff800000);
+            const uint32_t row = a.rows[r0 + t];
+            a.asn[row] = v.j;
+            a.costs[row] = nan0 ? __longlong_as_double(0x7ff8000000000000ll) : key_to_cost<SQRL2>(v.v);
+        }
+    }
+}
+
 int launch_assign_tiled(const AssignArgs &a, bool csr, bool pair, cudaStream_t st, bool tune) {
     if (a.n == 0) return MC_OK;
+    // a list of rows whose length the device knows: the kernel that the length calls for takes it,
+    // the other leaves at once
+    if (!csr && !pair && assign_few_takes(a, a.n_dev ? 1 : a.n)) {
+        k_assign_few<<<unsigned(umin64((a.n + 3) / 4, 152 * 4)), 128, a.d * sizeof(float4), st>>>(a), note_launch();
+        MC_CUDA_TRY(cudaGetLastError());
+        if (a.n <= kFewRows) return MC_OK;
+    }
     // 8x8 register tiles for SQRL2 with many centers, 4x4 otherwise
     const bool big = (a.msr == SQRL2 && a.kp % 128 == 0);
     if (!csr && pair && a.l1) {  // both are launched; one of them finds that the pass is the other's

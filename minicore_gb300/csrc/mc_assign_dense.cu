@@ -257,7 +257,10 @@ __global__ void __launch_bounds__(32 * WARPS, 12 / WARPS) k_assign_dense(const A
     using Cta = DenseCta<MSR, WARPS>;
     if (MSR == L1 && !l1_plain(a)) return;
     uint64_t nrows = a.n;
-    if (a.n_dev) nrows = umin64(nrows, *a.n_dev);
+    if (a.n_dev) {
+        nrows = umin64(nrows, *a.n_dev);
+        if (assign_few_takes(a, nrows)) return;
+    }
     Cta cta{a, dense_sm, dense_sm + Cta::PITCH * kx, kx, vec, 0, nrows};
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, tx = lane & 7, ty = lane >> 3;
     for (uint64_t tile = blockIdx.x; tile * Cta::BM < nrows; tile += gridDim.x) {

@@ -39,6 +39,12 @@ __device__ inline void best_merge_shfl(Best &b, int lanemask_xor) {
     }
 }
 
+// whether k_assign_few takes a list of nd rows: up to kFewRows, one resident wave of it
+constexpr uint64_t kFewRows = 2048;
+__host__ __device__ inline bool assign_few_takes(const AssignArgs &a, uint64_t nd) {
+    return a.msr == SQRL2 && a.rows && !a.dmode && a.d <= 2048 && nd <= kFewRows;
+}
+
 // final value of a pair: compare key (float) and cost (double) per measure
 template <int MSR>
 __device__ inline float finish_key(float acc) {
