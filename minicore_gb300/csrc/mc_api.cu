@@ -637,71 +637,16 @@ namespace {
 // ------------------------------------------------------------------------------------
 // Lloyd loop as one CUDA graph: [sort asn, check] -> while { centroids, assignment, objective,
 // stop rule, commit, sort asn, check }.  The stop rule of the host loop runs on the device
-// (k_loop_decide); the loop leaves the graph for the host only to finish (converged,
+// (loop_decide); the loop leaves the graph for the host only to finish (converged,
 // maxiter, cost rose -> revert, NaN center, bounded wait expired) or when a cluster is empty
 // (the D^2 restart of set_centroids_full_mean runs on the host, then the graph resumes).
 // Each kernel and its order are those of the host loop, so the results are identical.
 // ------------------------------------------------------------------------------------
-enum : int { LOOP_RUN = 0, LOOP_DONE = 1, LOOP_REVERT = 2, LOOP_EMPTY = 3, LOOP_NAN = 4, LOOP_TIMEOUT = 5 };
-
-struct LoopState {
-    float cost;                  // objective of the committed centers C
-    int reason;                  // LOOP_*
-    unsigned long long iternum;  // committed updates
-    unsigned long long maxiter;
-    double eps;
-    int commit;                  // the last decision copies Cw to C
-    int pad;
-};
-
-// graph != 0: the kernel runs inside the loop graph and also sets its while-condition h
-__global__ void k_loop_check_empty(const uint64_t *__restrict__ bucket_count, uint32_t k, LoopState *ls,
-                                   cudaGraphConditionalHandle h, int graph) {
-    __shared__ int any;
-    if (ls->reason != LOOP_RUN) return;  // same value for the whole block
-    if (threadIdx.x == 0) any = 0;
-    __syncthreads();
-    for (uint32_t c = threadIdx.x; c < k; c += blockDim.x)
-        if (bucket_count[c] == 0) any = 1;
-    __syncthreads();
-    if (threadIdx.x == 0 && any) {
-        ls->reason = LOOP_EMPTY;
-        if (graph) cudaGraphSetConditional(h, 0);
-    }
-}
-
-// the stop rule of the host loop (perform_hard_clustering, clustering/solve.h:98-175)
-__global__ void k_loop_decide(const double *__restrict__ cost_sum, const int *__restrict__ nan_flag,
-                              const int *__restrict__ tc_err, LoopState *ls, cudaGraphConditionalHandle h,
-                              int graph) {
-    ls->commit = 0;
-    if (*nan_flag) {
-        ls->reason = LOOP_NAN;
-        if (graph) cudaGraphSetConditional(h, 0);
-        return;
-    }
-    if (tc_err && *tc_err) {
-        ls->reason = LOOP_TIMEOUT;
-        if (graph) cudaGraphSetConditional(h, 0);
-        return;
-    }
-    const float newcost = float(*cost_sum);
-    if (newcost > ls->cost) {
-        ls->reason = LOOP_REVERT;
-        if (graph) cudaGraphSetConditional(h, 0);
-        return;
-    }
-    ls->commit = 1;
-    ls->iternum += 1;
-    const float oldcost = ls->cost;
-    ls->cost = newcost;
-    const double mx = double(newcost) < double(oldcost) ? double(oldcost) : double(newcost);
-    if (double(oldcost - newcost) < ls->eps * mx || ls->iternum > ls->maxiter) {
-        ls->reason = LOOP_DONE;
-        if (graph) cudaGraphSetConditional(h, 0);
-    } else {
-        if (graph) cudaGraphSetConditional(h, 1);
-    }
+// bucket sizes that the sort's own last CTA did not search (loop_empty)
+__global__ void k_loop_check_empty(const uint64_t *__restrict__ bucket_count, uint32_t k, const LoopCtl ctl) {
+    int any = 0;
+    for (uint32_t c = threadIdx.x; c < k; c += blockDim.x) any |= bucket_count[c] == 0;
+    if (__syncthreads_or(any) && threadIdx.x == 0) loop_empty(ctl);
 }
 
 __global__ void k_loop_commit(const LoopState *__restrict__ ls, float *C, const float *__restrict__ Cw, uint64_t m) {
@@ -724,11 +669,20 @@ struct CaptureGuard {  // ends an unfinished capture on the error path
 };
 
 // the loop's launch sequences (identical in the graph and in the fused host loop)
-int job_loop_pre(mc_job *j, LoopState *ls, cudaGraphConditionalHandle h, int graph) {
-    MC_TRY(launch_sort_by_key(j->asn.p, nullptr, j->M.n, j->k, j->sort, j->st));
-    k_loop_check_empty<<<1, 256, 0, j->st>>>(j->sort.bucket_count.p, j->k, ls, h, graph), note_launch();
+int job_loop_sort(mc_job *j, const LoopCtl &ctl) {
+    bool checked = false;
+    MC_TRY(launch_sort_by_key(j->asn.p, nullptr, j->M.n, j->k, j->sort, j->st, &ctl, &checked));
+    if (!checked) k_loop_check_empty<<<1, 256, 0, j->st>>>(j->sort.bucket_count.p, j->k, ctl), note_launch();
     MC_CUDA_TRY(cudaGetLastError());
     return MC_OK;
+}
+
+int job_loop_pre(mc_job *j, LoopState *ls, cudaGraphConditionalHandle h, int graph) {
+    LoopCtl ctl;
+    ctl.ls = ls;
+    ctl.h = h;
+    ctl.graph = graph;
+    return job_loop_sort(j, ctl);
 }
 
 // the centers of the current (sorted) assignment into Cw, no cluster empty
@@ -744,17 +698,19 @@ int job_loop_body(mc_job *j, LoopState *ls, cudaGraphConditionalHandle h, int gr
     const bool tc = j->M.kind == MC_DENSE_F32 && j->msr == SQRL2 && j->precision != MC_FP32;
     MC_TRY(job_update_centers(j));
     MC_TRY(job_assign_with(j, j->Cw.p, j->psum, false, nullptr, /*graph_mode=*/true));
+    LoopCtl ctl;
+    ctl.ls = ls;
+    ctl.nan_flag = j->flag.p;
+    ctl.tc_err = tc ? j->tc.err.p : nullptr;
+    ctl.h = h;
+    ctl.graph = graph;
     {
         DetInput in{j->w.p ? DET_F64_W : DET_F64, j->costs.p, nullptr, j->w.p, n};
-        MC_TRY(launch_det_sum(in, j->det_tmp.p, j->scal.p, st));
+        MC_TRY(launch_det_sum(in, j->det_tmp.p, j->scal.p, st, &ctl));
     }
-    k_loop_decide<<<1, 1, 0, st>>>(j->scal.p, j->flag.p, tc ? j->tc.err.p : nullptr, ls, h, graph), note_launch();
     const uint64_t m = uint64_t(k) * d;
     k_loop_commit<<<unsigned(umin64((m + 255) / 256, 1024)), 256, 0, st>>>(ls, j->C.p, j->Cw.p, m), note_launch();
-    MC_TRY(launch_sort_by_key(j->asn.p, nullptr, n, k, j->sort, st));
-    k_loop_check_empty<<<1, 256, 0, st>>>(j->sort.bucket_count.p, k, ls, h, graph), note_launch();
-    MC_CUDA_TRY(cudaGetLastError());
-    return MC_OK;
+    return job_loop_sort(j, ctl);
 }
 
 int job_build_loop_graph(mc_job *j) {

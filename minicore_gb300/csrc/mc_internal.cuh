@@ -251,7 +251,9 @@ __host__ __device__ inline uint64_t umin64(uint64_t a, uint64_t b) { return a < 
 // kernel launchers (defined in the .cu files)
 // ------------------------------------------------------------------------------------
 // reductions / draws (mc_reduce.cu)
-int launch_det_sum(const DetInput &in, double *chunk_tmp, double *out, cudaStream_t st);
+struct LoopCtl;
+// ctl: the kernel that finishes the sum also takes the loop's decision on it (mc_loop.cuh)
+int launch_det_sum(const DetInput &in, double *chunk_tmp, double *out, cudaStream_t st, const LoopCtl *ctl = nullptr);
 int launch_det_draw(const DetInput &in, double *chunk_tmp, const double *u_dev, double u_host, int use_dev_u,
                     const double *fallback_vals, uint64_t *out_idx, cudaStream_t st);
 // the same draw from the sums of 32-element blocks (n > 0); ticket: a zero that it leaves zero

@@ -62,7 +62,8 @@ __device__ void det_heap_build(double *T, uint64_t P, uint64_t G) {
     }
 }
 
-__global__ void __launch_bounds__(kDetThreads) k_det_final(double *tree, uint64_t P, uint64_t G, double *out) {
+__global__ void __launch_bounds__(kDetThreads) k_det_final(double *tree, uint64_t P, uint64_t G, double *out,
+                                                           const LoopCtl ctl) {
     __shared__ double sT[2 * kDetSmemLeaves];
     double *T = tree;
     if (P <= kDetSmemLeaves) {
@@ -70,8 +71,13 @@ __global__ void __launch_bounds__(kDetThreads) k_det_final(double *tree, uint64_
         T = sT;
     }
     det_heap_build(T, P, G);
-    if (threadIdx.x == 0) *out = T[1];
+    if (threadIdx.x == 0) {
+        *out = T[1];
+        if (ctl.ls) loop_decide(ctl, T[1]);
+    }
 }
+
+__global__ void k_loop_decide(const double *cost_sum, const LoopCtl ctl) { loop_decide(ctl, *cost_sum); }
 
 // Totals of 1024 consecutive elements, one warp each: loaded coalesced, turned through shared
 // memory so that each lane adds its 32 consecutive elements (31 adds per 32 elements, as
@@ -100,23 +106,25 @@ __global__ void __launch_bounds__(64) k_det_warps(DetInput in, double *leaves, u
     if (lane == 0) leaves[g] = t;
 }
 
-int launch_det_sum(const DetInput &in, double *chunk_tmp, double *out, cudaStream_t st) {
+int launch_det_sum(const DetInput &in, double *chunk_tmp, double *out, cudaStream_t st, const LoopCtl *ctl) {
+    const LoopCtl c = ctl ? *ctl : LoopCtl{};
     if (in.n > 0 && in.n <= kDetWarp * kDetSmemLeaves) {
         const uint64_t G = (in.n + kDetWarp - 1) / kDetWarp;
         uint64_t P = 1;
         while (P < G) P <<= 1;
         k_det_warps<<<unsigned((G + 1) / 2), 64, 0, st>>>(in, chunk_tmp + P, G), note_launch();
-        k_det_final<<<1, kDetThreads, 0, st>>>(chunk_tmp, P, G, out), note_launch();
+        k_det_final<<<1, kDetThreads, 0, st>>>(chunk_tmp, P, G, out, c), note_launch();
         MC_CUDA_TRY(cudaGetLastError());
         return MC_OK;
     }
     const uint64_t G = det_chunks(in.n), P = det_leaves(in.n);
     if (G == 0) {
         MC_CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(double), st));
+        if (ctl) k_loop_decide<<<1, 1, 0, st>>>(out, c), note_launch();
         return MC_OK;
     }
     k_det_chunks<<<unsigned(G), kDetThreads, 0, st>>>(in, chunk_tmp + P), note_launch();
-    k_det_final<<<1, kDetThreads, 0, st>>>(chunk_tmp, P, G, out), note_launch();
+    k_det_final<<<1, kDetThreads, 0, st>>>(chunk_tmp, P, G, out, c), note_launch();
     MC_CUDA_TRY(cudaGetLastError());
     return MC_OK;
 }
@@ -507,10 +515,12 @@ __global__ void k_sort_count(const uint32_t *__restrict__ keys, const uint32_t *
 // one CTA per key: exclusive scan of the key's tile counts (in place: per-tile offsets
 // relative to the bucket start) and the bucket total.  The last CTA to finish (ticket, which it
 // resets) also scans the totals into bucket_start and, with ch > 0, their chunks of ch rows into
-// chunk_start: in launches of their own the two scans took 2.6 us each, all latency.
+// chunk_start (in launches of their own the two scans took 2.6 us each, all latency), and looks for
+// empty buckets where the device-side loop wants to know.
 __global__ void __launch_bounds__(256) k_sort_key_scan(uint32_t *tile_counts, uint64_t ntiles, uint32_t k,
                                                        uint64_t *bucket_count, unsigned *ticket,
-                                                       uint64_t *bucket_start, uint64_t ch, uint64_t *chunk_start) {
+                                                       uint64_t *bucket_start, uint64_t ch, uint64_t *chunk_start,
+                                                       const LoopCtl ctl) {
     __shared__ uint64_t wsum[8], wsum2[8];
     __shared__ bool last;
     const uint32_t key = blockIdx.x;
@@ -553,9 +563,11 @@ __global__ void __launch_bounds__(256) k_sort_key_scan(uint32_t *tile_counts, ui
     // thread t: the keys [t q, t q + q)
     const uint32_t q = (k + 255) / 256, k0 = umin64(k, uint64_t(t) * q), k1 = umin64(k, uint64_t(k0) + q);
     uint64_t s1 = 0, s2 = 0;
+    int empty = 0;
     for (uint32_t i = k0; i < k1; ++i) {
         const uint64_t v = __ldcg(bucket_count + i);
         s1 += v;
+        empty |= v == 0;
         if (ch) s2 += (v + ch - 1) / ch;
     }
     uint64_t i1 = s1, i2 = s2;
@@ -565,7 +577,8 @@ __global__ void __launch_bounds__(256) k_sort_key_scan(uint32_t *tile_counts, ui
         if (lane >= off) i1 += v1, i2 += v2;
     }
     if (lane == 31) wsum[w] = i1, wsum2[w] = i2;
-    __syncthreads();
+    empty = __syncthreads_or(empty);
+    if (ctl.ls && empty && t == 0) loop_empty(ctl);
     uint64_t a1 = i1 - s1, a2 = i2 - s2;
     for (int i = 0; i < w; ++i) a1 += wsum[i], a2 += wsum2[i];
     for (uint32_t i = k0; i < k1; ++i) {
@@ -770,7 +783,7 @@ int launch_scan_ceil_div(const uint64_t *in, uint64_t *out, uint64_t m, uint64_t
 }
 
 int launch_sort_by_key(const uint32_t *keys, const uint32_t *keys2, uint64_t n, uint32_t k, SortWork &w,
-                       cudaStream_t st) {
+                       cudaStream_t st, const LoopCtl *ctl, bool *checked) {
     const uint64_t tile_rows = sort_tile_rows(n, k);
     const uint64_t ntiles = (n + tile_rows - 1) / tile_rows;
     MC_TRY(w.tile_counts.alloc(ntiles * k, st));
@@ -795,8 +808,10 @@ int launch_sort_by_key(const uint32_t *keys, const uint32_t *keys2, uint64_t n, 
     }
     if (ntiles)
         k_sort_key_scan<<<k, 256, 0, st>>>(w.tile_counts.p, ntiles, k, w.bucket_count.p, fused ? w.ticket.p : nullptr,
-                                           w.bucket_start.p, w.chunk_rows, w.chunk_start.p),
+                                           w.bucket_start.p, w.chunk_rows, w.chunk_start.p,
+                                           fused && ctl ? *ctl : LoopCtl{}),
             note_launch();
+    if (checked) *checked = fused && ctl;
     if (!fused)
         k_exclusive_scan_u64<<<1, 1024, 0, st>>>(w.bucket_count.p, w.bucket_start.p, k, 0), note_launch();
     if (ntiles) {

@@ -1,6 +1,7 @@
 // Sorting / centroid / statistics launchers (mc_reduce.cu).
 #pragma once
 #include "mc_internal.cuh"
+#include "mc_loop.cuh"
 
 namespace mc {
 
@@ -97,8 +98,9 @@ __device__ __forceinline__ unsigned long long c2_pack(float lo, float hi) {
     return r;
 }
 
+// ctl: also looks for empty buckets (loop_empty) where *checked comes back true
 int launch_sort_by_key(const uint32_t *keys, const uint32_t *keys2, uint64_t n, uint32_t k, SortWork &w,
-                       cudaStream_t st);
+                       cudaStream_t st, const LoopCtl *ctl = nullptr, bool *checked = nullptr);
 // chunk partials over CSR rows (mc_centroid_csr.cu); *done = false: not covered there
 int launch_centroid_chunks_csr(const CentroidArgs &a, SortWork &w, uint64_t max_chunks, uint64_t ch, cudaStream_t st,
                                bool *done);

@@ -29,3 +29,34 @@ def test_means_after_sort(n, k):
     assert np.array_equal(asn, lab)
     ref = np.stack([X[lab == c].astype(np.float64).sum(0) / np.count_nonzero(lab == c) for c in range(k)])
     assert np.array_equal(centers, ref.astype(np.float32))
+
+
+@pytest.mark.parametrize("k", [3, 256, 4096, 4097])
+@pytest.mark.parametrize("empty", [False, True])
+def test_loop_modes_agree_on_empty_clusters(k, empty):
+    """The search for empty clusters, in the sort's last block up to 4096 keys and in a launch of its
+    own past them, and the stop rule at the end of the objective's sum: the device loops run as the
+    host loop does, with a cluster that is empty from the start (last key) and without."""
+    import minicore_gb300 as mc
+    rng = np.random.default_rng(k)
+    C = (np.arange(k)[:, None] * 16 + np.zeros((1, 3))).astype(np.float32)
+    if empty:
+        C[k - 1] = -1e6
+    m = k - 1 if empty else k
+    lab = np.concatenate([np.arange(m), rng.integers(0, m, 2 * m)])
+    X = (lab[:, None] * 16 + rng.integers(-3, 4, size=(len(lab), 3))).astype(np.float32)
+    out = []
+    try:
+        for mode in (mc.LOOP_HOST, mc.LOOP_FUSED, mc.LOOP_GRAPH):
+            mc.loop_mode(mode)
+            job = mc.Job(X, C, msr=2, prior=0.0, seed=3)
+            job.run(eps=0.0, maxiter=6)
+            cen, asn, cost = np.empty_like(C), np.empty(len(X), np.uint32), np.empty(len(X), np.float64)
+            job.read(cen, asn, cost)
+            job.close()
+            out.append((cen, asn, cost))
+    finally:
+        mc.loop_mode(mc.LOOP_AUTO)
+    for o in out[1:]:
+        for x, y in zip(out[0], o):
+            assert np.array_equal(x, y)
