@@ -365,8 +365,9 @@ int job_assign_with(mc_job *j, const float *C, double prior_sum, bool force_exac
     const uint64_t n = j->M.n, d = j->M.d;
     const bool csr = j->M.kind == MC_CSR_F32;
     const bool tc = !csr && !force_exact && !dout && j->msr == SQRL2 && j->precision != MC_FP32;
-    // the norms, a sequential chain over the columns, serve the tensor-core pass only
-    MC_TRY(launch_center_sums(C, j->k, d, j->csum.p, tc ? j->cnorm.p : nullptr, j->st));
+    // the norms, a sequential chain over the columns, serve the tensor-core pass only, and SQRL2
+    // reads no sums (the prior does not enter it)
+    MC_TRY(launch_center_sums(C, j->k, d, j->msr == SQRL2 ? nullptr : j->csum.p, tc ? j->cnorm.p : nullptr, j->st));
     if (tc) {
         MC_TRY(tc_assign(j->tc, j->M.X, n, d, C, j->cnorm.p, j->k, j->precision, j->rownorm.p, j->asn.p,
                          j->costs.p, j->ctx->sms, j->st, &j->last_recheck, graph_mode));
@@ -471,8 +472,8 @@ __global__ void k_copy_row_csr(const float *vals, const uint32_t *idx, const uin
 
 // set_centroids_full_mean (centroid.h:649-779); returns 1 if a center was restarted
 // weighted means of the buckets into Cw (presorted: the counting sort of asn is current);
-// j->flag records a NaN center
-int job_launch_centroids(mc_job *j, const uint32_t *keys2, uint64_t extra, bool presorted) {
+// j->flag records a NaN center (clear: zeroed here; the device loop's stop rule leaves it zero)
+int job_launch_centroids(mc_job *j, const uint32_t *keys2, uint64_t extra, bool presorted, bool clear = true) {
     cudaStream_t st = j->st;
     Phase ph("centroid_update", st);
     CentroidArgs ca;
@@ -492,7 +493,7 @@ int job_launch_centroids(mc_job *j, const uint32_t *keys2, uint64_t extra, bool 
     ca.centers = j->Cw.p;
     ca.nan_flag = j->flag.p;
     ca.keep_bands = true;  // j->sort sorts rows of j->M only
-    MC_CUDA_TRY(cudaMemsetAsync(j->flag.p, 0, sizeof(int), st));
+    if (clear) MC_CUDA_TRY(cudaMemsetAsync(j->flag.p, 0, sizeof(int), st));
     return launch_centroids(ca, j->sort, st, presorted);
 }
 
@@ -678,6 +679,7 @@ int job_loop_sort(mc_job *j, const LoopCtl &ctl) {
 }
 
 int job_loop_pre(mc_job *j, LoopState *ls, cudaGraphConditionalHandle h, int graph) {
+    MC_CUDA_TRY(cudaMemsetAsync(j->flag.p, 0, sizeof(int), j->st));
     LoopCtl ctl;
     ctl.ls = ls;
     ctl.h = h;
@@ -686,9 +688,9 @@ int job_loop_pre(mc_job *j, LoopState *ls, cudaGraphConditionalHandle h, int gra
 }
 
 // the centers of the current (sorted) assignment into Cw, no cluster empty
-int job_update_centers(mc_job *j) {
+int job_update_centers(mc_job *j, bool clear) {
     if (l1_medians(j)) return job_l1_medians(j);
-    return job_launch_centroids(j, nullptr, 0, /*presorted=*/true);
+    return job_launch_centroids(j, nullptr, 0, /*presorted=*/true, clear);
 }
 
 int job_loop_body(mc_job *j, LoopState *ls, cudaGraphConditionalHandle h, int graph) {
@@ -696,7 +698,7 @@ int job_loop_body(mc_job *j, LoopState *ls, cudaGraphConditionalHandle h, int gr
     const uint64_t n = j->M.n, d = j->M.d;
     const uint32_t k = j->k;
     const bool tc = j->M.kind == MC_DENSE_F32 && j->msr == SQRL2 && j->precision != MC_FP32;
-    MC_TRY(job_update_centers(j));
+    MC_TRY(job_update_centers(j, /*clear=*/false));
     MC_TRY(job_assign_with(j, j->Cw.p, j->psum, false, nullptr, /*graph_mode=*/true));
     LoopCtl ctl;
     ctl.ls = ls;
@@ -728,7 +730,7 @@ int job_build_loop_graph(mc_job *j) {
     // space and the tensor-core path's FP32 rescan transform.  The centroid launch writes Cw,
     // which then takes the committed centers back (a restart on the host starts from Cw = C).
     MC_TRY(launch_sort_by_key(j->asn.p, nullptr, n, k, j->sort, st));
-    MC_TRY(job_update_centers(j));
+    MC_TRY(job_update_centers(j, /*clear=*/true));
     MC_CUDA_TRY(cudaMemcpyAsync(j->Cw.p, j->C.p, uint64_t(k) * d * sizeof(float), cudaMemcpyDeviceToDevice, st));
     if (tc) MC_TRY(j->tc.CT0.alloc(uint64_t(tiled_center_pad(k, false, SQRL2)) * d, st));
     CaptureGuard guard{st};

@@ -20,7 +20,8 @@ struct LoopState {
 
 struct LoopCtl {
     LoopState *ls = nullptr;  // null: the kernel decides nothing
-    const int *nan_flag = nullptr, *tc_err = nullptr;
+    int *nan_flag = nullptr;  // zero again after a decision
+    const int *tc_err = nullptr;
     cudaGraphConditionalHandle h{};
     int graph = 0;  // the kernel runs inside the loop graph and also sets its while-condition h
 };
@@ -38,6 +39,7 @@ __device__ inline void loop_decide(const LoopCtl &c, double cost_sum) {
     LoopState *ls = c.ls;
     ls->commit = 0;
     if (*c.nan_flag) {
+        *c.nan_flag = 0;
         ls->reason = LOOP_NAN;
         if (c.graph) cudaGraphSetConditional(c.h, 0);
         return;

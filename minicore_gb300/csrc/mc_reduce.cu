@@ -1288,7 +1288,7 @@ __global__ void __launch_bounds__(32) k_center_sums(const float *__restrict__ C,
         for (int u = 0; u < 8; ++u) {
             const int i = lane + 32 * u;
             if (i < cnt) {
-                s = s + double(x[u]);
+                if (csum) s = s + double(x[u]);
                 if (cnorm) t[i] = x[u];
             }
             x[u] = y[u];
@@ -1306,17 +1306,17 @@ __global__ void __launch_bounds__(32) k_center_sums(const float *__restrict__ C,
             __syncwarp();
         }
     }
-    double tot = 0.0;
+    if (csum) {
+        double tot = 0.0;
 #pragma unroll
-    for (int l = 0; l < 32; ++l) tot = tot + __shfl_sync(0xffffffffu, s, l);
-    if (lane == 0) {
-        csum[c] = tot;
-        if (cnorm) cnorm[c] = q;
+        for (int l = 0; l < 32; ++l) tot = tot + __shfl_sync(0xffffffffu, s, l);
+        if (lane == 0) csum[c] = tot;
     }
+    if (lane == 0 && cnorm) cnorm[c] = q;
 }
 
 int launch_center_sums(const float *C, uint32_t k, uint64_t d, double *csum, float *cnorm, cudaStream_t st) {
-    if (k == 0) return MC_OK;
+    if (k == 0 || (!csum && !cnorm)) return MC_OK;
     k_center_sums<<<k, 32, 0, st>>>(C, k, d, csum, cnorm), note_launch();
     MC_CUDA_TRY(cudaGetLastError());
     return MC_OK;
