@@ -1510,9 +1510,18 @@ static int job_create_impl(mc_context *ctx, const mc_matrix *X, const float *cen
             MC_TRY(launch_row_scalars(j->rowsum.p, n, d, j->pv, j->rsi.p, j->rinc.p, st));
         }
     }
-    if (msr == L1 && j->pair && j->M.kind == MC_DENSE_F32) {
+    if (msr == L1 && j->pair && j->M.kind == MC_DENSE_F32 && l1_dense_pays(n, d, k)) {
+        L1Stat rows;
         MC_TRY(j->l1stat.alloc(1, st));
         MC_TRY(launch_l1_row_stat(j->M.X, n * d, j->rowsum.p, n, j->l1stat.p, st));
+        MC_CUDA_TRY(cudaMemcpyAsync(&rows, j->l1stat.p, sizeof(rows), cudaMemcpyDeviceToHost, st));
+        MC_TRY(sync(st));
+        double xsum;
+        float xmin;
+        std::memcpy(&xsum, &rows.xsum, sizeof(xsum));
+        std::memcpy(&xmin, &rows.xmin, sizeof(xmin));
+        // rows that rule the plain form out by themselves keep the pair kernel alone
+        if (!l1_plain_bounds(xsum + 2.0 * std::fabs(j->psum), j->prior, xmin)) j->l1stat.release();
     }
     j->sort.chunk_rows = centroid_chunk_rows(j->M.kind == MC_CSR_F32);
     j->sparse_path = j->M.kind == MC_CSR_F32 && !j->pair && (msr != JSD || j->ngrp > 0);

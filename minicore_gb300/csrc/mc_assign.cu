@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(256) k_assign_tiled(AssignArgs a) {
     }
 
     // L1 pairs over dense rows: a resident grid strides over the tiles, so that a pass that is
-    // k_assign_dense's costs two CTAs per SM that leave at once, not one per tile (17 -> 4 us, 100,000 rows)
+    // k_assign_dense's costs kPairCtas CTAs per SM that leave at once, not one per tile
     constexpr bool kStride = MSR == L1 && PAIR && !CSR;
     do {
     float rpv = a.pv;
@@ -1276,13 +1276,18 @@ int launch_assign_l1_union(const AssignArgs &a, const float *C, float *work, int
     return MC_OK;
 }
 
+// CTAs of the L1 pair kernel that an SM holds (48 registers a thread).  100,000 x 64, k = 50: where the
+// prior changes terms after all two per SM took 178 us and five 145; where it does not, and they leave
+// at once, 92 and 94
+constexpr unsigned kPairCtas = 5;
+
 template <int MSR, bool CSR>
 static int tiled_t(const AssignArgs &a, bool pair, bool big, cudaStream_t st, bool tune) {
     if (pair) {
         constexpr int BM = 32;
         const uint64_t tiles = (a.n + BM - 1) / BM;
         const bool stride = MSR == L1 && !CSR && a.l1;
-        k_assign_tiled<MSR, true, 2, 2, CSR><<<unsigned(stride ? umin64(tiles, 152 * 2) : tiles), 256, 0, st>>>(a),
+        k_assign_tiled<MSR, true, 2, 2, CSR><<<unsigned(stride ? umin64(tiles, 152 * kPairCtas) : tiles), 256, 0, st>>>(a),
             note_launch();
     } else if (big) {
         // SQRL2 with kp % 128 == 0: 8x8 register tiles (128 rows per CTA) or 4x4 (64 rows), dense
@@ -1341,7 +1346,7 @@ __global__ void __launch_bounds__(256) k_l1_stat(const float *__restrict__ v, ui
 
 static int l1_stat(const float *v, uint64_t m, const double *sums, uint64_t n, unsigned *vmin, unsigned long long *smax,
                    cudaStream_t st) {
-    MC_CUDA_TRY(cudaMemsetAsync(vmin, 0x7f, sizeof(unsigned), st));  // a NaN pattern: above every magnitude
+    MC_CUDA_TRY(cudaMemsetAsync(vmin, 0x7f, sizeof(unsigned), st));  // 3.4e38: no nonzero below it
     MC_CUDA_TRY(cudaMemsetAsync(smax, 0, sizeof(unsigned long long), st));
     k_l1_stat<<<unsigned(umin64((m + 1023) / 1024, 152 * 4)), 256, 0, st>>>(v, m, sums, n, vmin, smax), note_launch();
     MC_CUDA_TRY(cudaGetLastError());

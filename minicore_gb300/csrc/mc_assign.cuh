@@ -12,6 +12,26 @@ struct L1Stat {
     unsigned xmin, cmin;
 };
 
+// L1 in pair mode adds the pair's pv to both values of a column: at most
+// 7.0069e-42 (row sum + center sum), or the prior itself.  Where every nonzero magnitude exceeds
+// 2^26 times that, v + pv rounds to v for v != 0, |pv - v| rounds to |v| and |pv - pv| is 0, so
+// each term is exactly |c - x| of the raw values.  (A NaN sum or bound fails the comparison.)
+__host__ __device__ inline bool l1_plain_bounds(double sums, double prior, float mn) {
+    double pv = 7.0069e-42 * sums * 1.0001 + 1e-44;
+    if (prior > pv) pv = prior;
+    return double(mn) > pv * 67108864.0;
+}
+
+// Which dense L1 pair passes are offered to k_assign_dense: that launch, the bounds of the centers and
+// the pair kernel's CTAs that leave cost some 10 us, and below 38,912 rows its 128-row tiles leave SMs
+// idle.  Assignment in us, offered / the pair kernel alone (n x d, k; padded: n d times k rounded up to
+// the pair kernel's 32): 300,000 x 20, k = 10 (1.9e8): 65 / 95; 40,000 x 64, k = 50 (1.6e8): 57 / 62;
+// 100,000 x 64, k = 50 (4.1e8): 92 / 117; 40,000 x 32, k = 50 (8.2e7): 44 / 40; 100,000 x 20, k = 10
+// (6.4e7): 40 / 42; 20,000 x 64, k = 50 (8.2e7): 49 / 41.
+inline bool l1_dense_pays(uint64_t n, uint64_t d, uint32_t k) {
+    return n > 128 * 152 * 2 && double(n) * double(d) * double((uint64_t(k) + 31) / 32 * 32) >= 1.2e8;
+}
+
 struct AssignArgs {
     int msr = SQRL2;
     uint64_t n = 0, d = 0;

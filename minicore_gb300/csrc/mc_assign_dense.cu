@@ -324,7 +324,7 @@ int launch_assign_dense(const AssignArgs &a, cudaStream_t st, bool *done) {
     if (a.msr == SQRL2) return wide ? dense_launch_w<SQRL2, 4>(a, st) : dense_launch_w<SQRL2, 2>(a, st);
     if (a.msr == MKL && a.k > 64) return wide ? dense_launch_w<MKL, 4>(a, st) : dense_launch_w<MKL, 2>(a, st);
     // L1 in pair mode where its terms are plain differences (l1_plain): 100,000 x 64, k = 50:
-    // 105 -> 67 us (and 4 us for the CTAs of k_assign_tiled that leave at once)
+    // 105 -> 67 us (and 6 us for the CTAs of k_assign_tiled that leave at once); which sizes: l1_dense_pays
     if (a.msr == L1 && a.l1) return wide ? dense_launch_w<L1, 4>(a, st) : dense_launch_w<L1, 2>(a, st);
     *done = false;
     return MC_OK;

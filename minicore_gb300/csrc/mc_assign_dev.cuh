@@ -75,18 +75,13 @@ __device__ inline void row_xform(float x, float pv, float rsi, float rinc, float
     }
 }
 
-// L1 in pair mode adds the pair's pv to both values of a column: at most
-// 7.0069e-42 (row sum + center sum), or the prior itself.  Where every nonzero magnitude exceeds
-// 2^26 times that, v + pv rounds to v for v != 0, |pv - v| rounds to |v| and |pv - pv| is 0, so
-// each term is exactly |c - x| of the raw values.  (A NaN sum or bound fails the comparison.)
+// plain differences, by the rows' and the centers' bounds (l1_plain_bounds)
 __device__ inline bool l1_plain(const AssignArgs &a) {
     const L1Stat &t = *a.l1;
     const double sums = __longlong_as_double((long long)t.xsum) + __longlong_as_double((long long)t.csum) +
                         2.0 * fabs(a.prior_sum);
-    double pv = 7.0069e-42 * sums * 1.0001 + 1e-44;
-    if (a.prior > pv) pv = a.prior;
     const float mn = fminf(__uint_as_float(t.xmin), __uint_as_float(t.cmin));
-    return double(mn) > pv * 67108864.0;
+    return l1_plain_bounds(sums, a.prior, mn);
 }
 
 }  // namespace mc

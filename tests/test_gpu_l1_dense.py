@@ -66,3 +66,26 @@ def test_soft_clustering_edges(n, d, k, weighted):
     assert r["numiter"] == o["numiter"]
     assert np.allclose(r["centers"], o["centers"], rtol=1e-4, atol=1e-5)
     assert np.allclose(r["asn"], o["asn"], atol=1e-5)
+
+
+@pytest.mark.parametrize("rows,centers", [(1.0, 1.0), (1e-41, 1.0), (1.0, 1e-41)])
+@pytest.mark.parametrize("n,d,k", [(38912, 80, 33), (38913, 80, 33), (50001, 41, 64), (100001, 15, 66)])
+def test_l1_assignment_of_many_rows(rows, centers, n, d, k):
+    """Sizes from which plain differences have a kernel of their own: taken, ruled out by the rows and
+    ruled out by the centers alone (the pair kernel's CTAs then walk several tiles each)."""
+    import minicore_gb300 as mc
+    import oracle
+    rng = np.random.default_rng(n + k)
+    X = rng.integers(0, 5, (n, d)).astype(np.float32)
+    C = X[rng.choice(n, k, replace=False)].copy()
+    X[::3] *= np.float32(rows)
+    C[::2] *= np.float32(centers)
+    C[0, ::2] += np.float32(3.0)
+    job = mc.Job(X, C, msr=0, prior=0.0)
+    job.assign()
+    asn, cost = np.empty(n, np.uint32), np.empty(n, np.float64)
+    job.read(None, asn, cost)
+    job.close()
+    oasn, ocost = oracle.assign(X, C, 0, 0.0)
+    assert np.array_equal(asn, oasn)
+    assert np.array_equal(cost, ocost)
