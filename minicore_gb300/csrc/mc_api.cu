@@ -272,7 +272,8 @@ struct mc_job {
     DBuf<double> ztab;
     DBuf<float> jlogs;      // centers' a and a log a
     uint32_t ngrp = 0;
-    // rows listed by group, for k_assign_jsd_groups (jgroups: it takes this job's passes)
+    // rows listed by group, for k_assign_jsd_groups (jgroups: it takes this job's passes of as many
+    // centers as pay)
     bool jgroups = false;
     JsdGroupWork jgw;
     SortWork sort;
@@ -415,7 +416,9 @@ int job_assign_with(mc_job *j, const float *C, double prior_sum, bool force_exac
         a.consts = j->consts.p;
     }
     MC_TRY(launch_prep_centers(a, C, j->pair, sparse, j->st));
-    if (j->l1stat.p) {
+    // (these rules look at the centers of this pass: the restarts of the coreset minibatch take fewer
+    // than the job's)
+    if (j->l1stat.p && l1_dense_pays(n, d, j->k)) {
         MC_TRY(launch_l1_center_stat(C, uint64_t(j->k) * d, j->csum.p, j->k, j->l1stat.p, j->st));
         a.l1 = j->l1stat.p;
     }
@@ -428,7 +431,8 @@ int job_assign_with(mc_job *j, const float *C, double prior_sum, bool force_exac
     }
     if (sparse) {
         Phase ph("assign_csr_sparse", j->st);
-        if (j->jgroups) {
+        if (j->jgroups && jsd_groups_pay(n, d, j->k, j->M.nnz, j->ngrp)) {
+            Phase pg("assign_jsd_groups", j->st);
             JsdGroups g;
             g.nbucket = j->ngrp + 1;
             g.perm = j->jgw.sort.perm.p;

@@ -267,6 +267,8 @@ bool jsd_groups_pay(uint64_t n, uint64_t d, uint32_t k, uint64_t nnz, uint32_t n
 
 int launch_assign_jsd_groups(const AssignArgs &a, const JsdGroups &jg, cudaStream_t st) {
     if (a.n == 0) return MC_OK;
+    // a band's columns are staged 64 centers at a time, which CT0's padding has to hold
+    if (a.kp % 64) return fail(MC_EINVAL, "JSD row groups: the centers are not padded to 64");
     MC_CUDA_TRY(cudaFuncSetAttribute(k_assign_jsd_groups, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kJsdSmem)));
     // slabs: at most one partial one per group
     const uint64_t slabs = a.n / kJsdSlab + jg.nbucket;
