@@ -1290,16 +1290,21 @@ static int tiled_t(const AssignArgs &a, bool pair, bool big, cudaStream_t st, bo
         k_assign_tiled<MSR, true, 2, 2, CSR><<<unsigned(stride ? umin64(tiles, 152 * kPairCtas) : tiles), 256, 0, st>>>(a),
             note_launch();
     } else if (big) {
-        // SQRL2 with kp % 128 == 0: 8x8 register tiles (128 rows per CTA) or 4x4 (64 rows), dense
-        // rows k_assign_dense or 8x8; same per-pair arithmetic, so the autotuner may pick either
-        const std::string key = std::string("dense_sqrl2|") + (CSR ? "csr" : "dense") + "|k" +
-                                std::to_string(a.kp) + "|d" + tune_bucket(a.d) + "|n" + tune_bucket(a.n);
-        return tune_launch(key, 2, 0, st, tune, [&](int v) -> int {
-            if (!CSR && v == 0) {
-                bool done = false;
-                return launch_assign_dense(a, st, &done);
-            }
-            if (v == (CSR ? 0 : 1))
+        // SQRL2 with kp % 128 == 0: 8x8 register tiles (128 rows per CTA), 4x4 (64 rows) or, for dense
+        // rows of 48 columns and more, k_assign_dense; same per-pair arithmetic, so the autotuner may pick
+        // any, and where it may not time the rule of assign_dense_pays decides.  For dense rows the key
+        // holds k and d in the steps of that kernel (its times relative to the others' turn within a power
+        // of two), and the number of variants, as in decisions of another numbering the key had none.
+        const int nvar = !CSR && a.d >= 48 ? 3 : 2;
+        const std::string key =
+            CSR ? "dense_sqrl2|csr|k" + std::to_string(a.kp) + "|d" + tune_bucket(a.d) + "|n" + tune_bucket(a.n)
+                : "dense_sqrl2|dense|k" + std::to_string((a.k + 15) / 16 * 16) + "|d" +
+                      std::to_string((a.d + 15) / 16 * 16) + "|n" + tune_bucket(a.n) + "|v" + std::to_string(nvar);
+        const int rule = nvar == 3 && assign_dense_pays(a) ? 2 : 0;
+        return tune_launch(key, nvar, rule, st, tune, [&](int v) -> int {
+            if constexpr (!CSR)
+                if (v == 2) return launch_assign_dense(a, st);
+            if (v == 0)
                 k_assign_tiled<MSR, false, 8, 8, CSR><<<unsigned((a.n + 127) / 128), 256, 0, st>>>(a), note_launch();
             else
                 k_assign_tiled<MSR, false, 4, 4, CSR><<<unsigned((a.n + 63) / 64), 256, 0, st>>>(a), note_launch();
@@ -1434,15 +1439,9 @@ int launch_assign_tiled(const AssignArgs &a, bool csr, bool pair, cudaStream_t s
     }
     // 8x8 register tiles for SQRL2 with many centers, 4x4 otherwise
     const bool big = (a.msr == SQRL2 && a.kp % 128 == 0);
-    if (!csr && pair && a.l1) {  // both are launched; one of them finds that the pass is the other's
-        bool done = false;
-        MC_TRY(launch_assign_dense(a, st, &done));
-    }
-    if (!csr && !pair && !big) {
-        bool done = false;
-        MC_TRY(launch_assign_dense(a, st, &done));
-        if (done) return MC_OK;
-    }
+    // both are launched; one of them finds that the pass is the other's
+    if (!csr && pair && a.l1) MC_TRY(launch_assign_dense(a, st));
+    if (!csr && !pair && !big && assign_dense_pays(a)) return launch_assign_dense(a, st);
     switch (a.msr) {
         case SQRL2:
             return csr ? tiled_t<SQRL2, true>(a, pair, big, st, tune) : tiled_t<SQRL2, false>(a, pair, big, st, tune);

@@ -23,13 +23,15 @@ __host__ __device__ inline bool l1_plain_bounds(double sums, double prior, float
 }
 
 // Which dense L1 pair passes are offered to k_assign_dense: that launch, the bounds of the centers and
-// the pair kernel's CTAs that leave cost some 10 us, and below 38,912 rows its 128-row tiles leave SMs
-// idle.  Assignment in us, offered / the pair kernel alone (n x d, k; padded: n d times k rounded up to
-// the pair kernel's 32): 300,000 x 20, k = 10 (1.9e8): 65 / 95; 40,000 x 64, k = 50 (1.6e8): 57 / 62;
-// 100,000 x 64, k = 50 (4.1e8): 92 / 117; 40,000 x 32, k = 50 (8.2e7): 44 / 40; 100,000 x 20, k = 10
-// (6.4e7): 40 / 42; 20,000 x 64, k = 50 (8.2e7): 49 / 41.
+// the pair kernel's CTAs that leave cost some 17 us, and below 38,912 rows its 128-row tiles leave SMs
+// idle.  Assignment in us, offered / the pair kernel alone, over the grid named at assign_dense_pays
+// (n x d, k; work: n d times k rounded up to the pair kernel's 32): up to 16 centers, which that kernel
+// pads to 32, it pays from a work of 1.2e8 (300,000 x 20, k = 10: 65 / 95); else from 4e8 and 32 columns
+// (100,000 x 64, k = 50: 92 / 117), below which it loses (60,000 x 32, k = 64, 1.2e8: 64 / 54;
+// 75,000 x 50, k = 32, 1.2e8: 63 / 54; 60,000 x 16, k = 1000, 9.8e8: 406 / 347)
 inline bool l1_dense_pays(uint64_t n, uint64_t d, uint32_t k) {
-    return n > 128 * 152 * 2 && double(n) * double(d) * double((uint64_t(k) + 31) / 32 * 32) >= 1.2e8;
+    const double work = double(n) * double(d) * double((uint64_t(k) + 31) / 32 * 32);
+    return n > 128 * 152 * 2 && (k <= 16 ? work >= 1.2e8 : d >= 32 && work >= 4e8);
 }
 
 struct AssignArgs {
@@ -82,8 +84,10 @@ int launch_row_scalars(const double *rowsum, uint64_t n, uint64_t d, float pv, f
 // tune: the autotuner may time kernel variants on the first call for a shape (callers that
 // must not synchronise or allocate pass false)
 int launch_assign_tiled(const AssignArgs &a, bool csr, bool pair, cudaStream_t st, bool tune = true);
-// dense rows, constant prior (mc_assign_dense.cu); *done = false: not covered there
-int launch_assign_dense(const AssignArgs &a, cudaStream_t st, bool *done);
+// dense rows in chunks of 64 centers (mc_assign_dense.cu): SQRL2, MKL with a constant prior, plain L1; and
+// whether it rather than k_assign_tiled takes a pass
+int launch_assign_dense(const AssignArgs &a, cudaStream_t st);
+bool assign_dense_pays(const AssignArgs &a);
 int launch_assign_sparse(const AssignArgs &a, cudaStream_t st, int sms, bool tune = true);
 // L1 over CSR rows in pair mode (prior 0): a walk over the union of nonzero columns,
 // bit-identical to the tiled kernel; work: l1_union_work_entries(k, d) floats

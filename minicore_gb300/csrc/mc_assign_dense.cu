@@ -269,9 +269,11 @@ __global__ void __launch_bounds__(32 * WARPS, 12 / WARPS) k_assign_dense(const A
         best_init(best);
         bool have_rows = false;
         uint32_t c = 0;
-        while (c < a.k) {  // 64, 32 or 16 centers at a time
+        // 64, 32 or 16 centers at a time; 33 to 48 go as 64, which takes less time than 32 and 16 (MKL
+        // 100,000 x 160, k = 100: 376 us as 64 + 32 + 16, 315 as 64 + 64)
+        while (c < a.k) {
             const uint32_t left = a.k - c;
-            if (left > 48) {
+            if (left > 32) {
                 cta.template chunk<8>(c, have_rows, best);
                 c += 64;
             } else if (left > 16) {
@@ -292,11 +294,16 @@ __global__ void __launch_bounds__(32 * WARPS, 12 / WARPS) k_assign_dense(const A
     }
 }
 
+// columns per load of a row
+static int row_vec(const AssignArgs &a) {
+    const uintptr_t xp = reinterpret_cast<uintptr_t>(a.X);
+    return a.d % 4 == 0 && xp % 16 == 0 ? 4 : a.d % 2 == 0 && xp % 8 == 0 ? 2 : 1;
+}
+
 template <int MSR, int WARPS>
 static int dense_launch_w(const AssignArgs &a, cudaStream_t st) {
     const int kx = int(umin64((a.d + kStep - 1) / kStep * kStep, kDenseCols));
-    const uintptr_t xp = reinterpret_cast<uintptr_t>(a.X);
-    const int vec = a.d % 4 == 0 && xp % 16 == 0 ? 4 : a.d % 2 == 0 && xp % 8 == 0 ? 2 : 1;
+    const int vec = row_vec(a);
     constexpr int BM = WARPS * kDenseRowsPerWarp;
     auto smem_of = [](int cols) { return (size_t(BM + 4) * cols + 2 * DenseTile<MSR>::CBUF) * sizeof(float); };
     auto kern = k_assign_dense<MSR, WARPS>;
@@ -311,23 +318,45 @@ static int dense_launch_w(const AssignArgs &a, cudaStream_t st) {
     return MC_OK;
 }
 
-// Which calls come here (the others: k_assign_tiled), from measured pairs (new / k_assign_tiled):
-// SQRL2 300,001 x 100, k = 200: 528 / 700 us; 100,000 x 101, k = 40: 63 / 80; 200,000 x 16, k = 8:
-// 22 / 32; 10,000 x 50, k = 25: 13.5 / 13.3.  Rows of more than kDenseCols columns against many
-// centers are loaded once per chunk of 64 (30,000 x 256, k = 1000: 976 / 828), so the autotuner
-// chooses where k is padded to 128.  MKL 100,000 x 64, k = 200: 189 / 257, k = 100: 115 / 130,
-// 20,000 rows, k = 50: 25.5 / 22.2, so from 65 centers on; Hellinger (a square root per row entry and
-// CTA, k = 100: 120 / 111) and JSD (a logarithm per pair) do not come here.
-int launch_assign_dense(const AssignArgs &a, cudaStream_t st, bool *done) {
-    *done = true;
-    const bool wide = a.n > 128 * 152 * 2;  // 128 rows per CTA, 64 where that leaves SMs without a tile
-    if (a.msr == SQRL2) return wide ? dense_launch_w<SQRL2, 4>(a, st) : dense_launch_w<SQRL2, 2>(a, st);
-    if (a.msr == MKL && a.k > 64) return wide ? dense_launch_w<MKL, 4>(a, st) : dense_launch_w<MKL, 2>(a, st);
-    // L1 in pair mode where its terms are plain differences (l1_plain): 100,000 x 64, k = 50:
-    // 105 -> 67 us (and 6 us for the CTAs of k_assign_tiled that leave at once); which sizes: l1_dense_pays
-    if (a.msr == L1 && a.l1) return wide ? dense_launch_w<L1, 4>(a, st) : dense_launch_w<L1, 2>(a, st);
-    *done = false;
-    return MC_OK;
+// Which passes come here (n x d rows, k centers) and which go to k_assign_tiled, from both kernels' times
+// (here / k_assign_tiled, us) over 17 row counts of 3,000 to 1,000,000, 21 column counts of 8 to 256 and
+// 16 center counts of 8 to 1000; at the worst point of that grid the rule loses 4 %.  What decides:
+//  * k_assign_tiled pads k to 64 (128 from 65 on), a chunk here to 16, 32 or 64: up to 32 centers this
+//    kernel gains even where it runs less well (SQRL2 150,000 x 16, k = 8: 18 / 28; 100,000 x 64,
+//    k = 32: 30 / 55);
+//  * a chunk starts with a barrier and a fetch and ends with the argmin over its centers, which few
+//    columns do not pay for (SQRL2 300,000 x 16, k = 64: 64 / 49; x 50, k = 128: 208 / 190);
+//  * twelve warps per SM fit up to some 112 columns, eight up to 176 (MKL, whose center tile is twice as
+//    large: 64 and 144), then four (SQRL2 300,000 x 192, k = 128: 758 / 671; MKL 39,500 x 256, k = 128:
+//    264 / 247; at 144: 119 / 141); past kDenseCols the rows are also loaded, and MKL's logarithms taken, again for every
+//    64 centers (SQRL2 300,000 x 256, k = 128: 1043 / 890);
+//  * odd columns are loaded four bytes at a time (SQRL2 60,000 x 97, k = 100: 95 / 90; x 96: 82 / 86).
+// Hellinger (a square root per row entry and CTA, k = 100: 120 / 111) and JSD (a logarithm per pair) do
+// not come here, nor does MKL up to 64 centers.
+bool assign_dense_pays(const AssignArgs &a) {
+    const uint64_t n = a.n, d = a.d;
+    const uint32_t k = a.k;
+    const bool odd = row_vec(a) == 1;
+    if (a.msr == MKL) return k > 64 && d >= (odd ? 112 : 64) && d <= (k > 128 ? 192 : 144);
+    if (a.msr != SQRL2) return false;
+    if (k <= 16) return d >= 16;
+    if (k <= 32) return d >= 48 || (d >= 32 && n >= 12000);
+    if (k > 64) return !odd && d >= 112 && d <= 176;
+    if (odd) return d >= 112 && d <= 176;
+    if (d > 176) return n > 128 * 152 * 2;
+    return d >= 72 || (d >= 64 && n >= 75000);
+}
+
+int launch_assign_dense(const AssignArgs &a, cudaStream_t st) {
+    // 128 rows per CTA; 64 where a tile of 128 rows leaves room for one CTA per SM (SQRL2 300,000 x 256,
+    // k = 64: 457 / 559 us)
+    switch (a.msr) {
+        case SQRL2: return a.d <= 176 ? dense_launch_w<SQRL2, 4>(a, st) : dense_launch_w<SQRL2, 2>(a, st);
+        case MKL: return dense_launch_w<MKL, 4>(a, st);
+        // L1 in pair mode where its terms are plain differences (l1_plain); which sizes: l1_dense_pays
+        case L1: return dense_launch_w<L1, 4>(a, st);
+        default: return fail(MC_EUNSUPPORTED, "k_assign_dense does not cover this measure");
+    }
 }
 
 }  // namespace mc

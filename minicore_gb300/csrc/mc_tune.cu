@@ -2,8 +2,8 @@
 //
 // Tuned families (all variants bit-identical by construction):
 //   csr_sparse   k_assign_sparse nonzero batch size (8, 4, 16)
-//   dense_sqrl2  SQRL2 FP32 assignment (large shapes: k_assign_dense or k_assign_tiled 8x8; small
-//                ones: k_assign_tiled 8x8 / 128 rows or 4x4 / 64 rows)
+//   dense_sqrl2  SQRL2 FP32 assignment from 65 centers on: k_assign_tiled 8x8 / 128 rows or 4x4 /
+//                64 rows, and for dense rows of 48 columns and more k_assign_dense
 //   kmpp_dense   kmeans++ distance update (cp.async-staged rows, direct loads)
 // Keys carry the device (compute capability and SM count) and the shape bucket.  Decisions
 // live in a process-wide table, loaded from and appended to a cache file:
