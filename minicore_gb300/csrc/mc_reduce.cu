@@ -1328,8 +1328,11 @@ int launch_center_sums(const float *C, uint32_t k, uint64_t d, double *csum, flo
 // warps) per (cluster, 32 columns): the largest weight of the cluster, then per
 // column the smallest value among the rows that carry it.
 // ------------------------------------------------------------------------------------
+// keys in the order of the values (NaN past infinity on its sign's side).  The bits come by an opaque
+// move: seen through, the compiler may form u | 0x80000000 as -|v|, whose NaN is 0x7fffffff, the key of -0
 __device__ __forceinline__ uint32_t f2ord(float v) {
-    const uint32_t u = __float_as_uint(v);
+    uint32_t u;
+    asm("mov.b32 %0, %1;" : "=r"(u) : "f"(v));
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 __device__ __forceinline__ float ord2f(uint32_t k) {
