@@ -333,9 +333,13 @@ __device__ __forceinline__ double alias_scale(uint64_t n, const double *S) {
     return sm_scale;
 }
 
-// a < b for values that are not negative (nor NaN): their bits as integers, because FP64
-// comparisons run at about two lanes per SM and clock
-__device__ __forceinline__ bool nn_less(double a, double b) { return __double_as_longlong(a) < __double_as_longlong(b); }
+// The order of values that are not negative, as integers (their bits), because FP64 comparisons run at
+// about two lanes per SM and clock.  A NaN comes before all of them: sums of excesses are NaN from the
+// first infinite probability on (its share of an infinite total).
+__device__ __forceinline__ long long nn_key(double v) {
+    const long long b = __double_as_longlong(v);
+    return (b & 0x7fffffffffffffffll) > 0x7ff0000000000000ll ? -1ll : b;
+}
 
 __global__ void k_alias_flags(const float *probs, uint64_t n, const double *S, uint64_t *light_flag) {
     const double scale = alias_scale(n, S);
@@ -365,11 +369,11 @@ __global__ void k_alias_light(const float *probs, uint64_t n, const double *S, c
                               uint32_t *alias_tab) {
     const double scale = alias_scale(n, S);
     for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < nl; i += gridDim.x * uint64_t(blockDim.x)) {
-        const double Di = D[i];
+        const long long Di = nn_key(D[i]);
         uint64_t lo = 0, hi = nh;
         while (lo < hi) {
             const uint64_t mid = (lo + hi) >> 1;
-            if (nn_less(E[mid + 1], Di)) lo = mid + 1; else hi = mid;
+            if (nn_key(E[mid + 1]) < Di) lo = mid + 1; else hi = mid;
         }
         const uint64_t j = lo < nh ? lo : nh - 1;
         const uint32_t li = L[i];
@@ -383,11 +387,11 @@ __global__ void k_alias_heavy(const uint32_t *H, uint64_t nh, uint64_t nl, const
     for (uint64_t j = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; j < nh; j += gridDim.x * uint64_t(blockDim.x)) {
         uint64_t i = nl;
         if (j + 1 < nh) {
-            const double Ej = E[j + 1];
-            uint64_t lo = 0, hi = nl;
+            const long long Ej = nn_key(E[j + 1]);
+            uint64_t lo = Ej < 0 ? nl : 0, hi = nl;  // no sum of lights is past a NaN
             while (lo < hi) {
                 const uint64_t mid = (lo + hi) >> 1;
-                if (nn_less(Ej, D[mid + 1])) hi = mid; else lo = mid + 1;
+                if (Ej < nn_key(D[mid + 1])) hi = mid; else lo = mid + 1;
             }
             i = lo;
         }
