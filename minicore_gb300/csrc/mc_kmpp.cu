@@ -273,6 +273,8 @@ __global__ void __launch_bounds__(256) k_kmpp_csr(const KmppArgs a, int first, u
             s.rhinc = __shfl_sync(0xffffffffu, sm.rhinc, r);
             const uint64_t pb = __shfl_sync(0xffffffffu, pbm, r), pe = __shfl_sync(0xffffffffu, pem, r);
             float acc = 0.f;
+            // (JSD, 20,000 x 20,000, a round: 2.9 ms without the loads of four columns in flight, 1.9 with)
+#pragma unroll 4
             for (uint64_t j = lane; j < a.d; j += 32) kp_elem<MSR>(acc, a.cbuf[j], 0.f, s);
             for (uint64_t p = pb + lane; p < pe; p += 32) {
                 const float cj = a.cbuf[a.idx[p]];
@@ -475,16 +477,17 @@ __device__ __forceinline__ void kp_csr_rows(const KmppArgs &a, int first, uint32
         }
         float accm = 0.f;    // lane l: row g0 + l's float sum
         double bsumm = 0.0;  // lane l: row g0 + l's FP64 sum (Hellinger)
-        const unsigned todo = __ballot_sync(0xffffffffu, go), fastb = __ballot_sync(0xffffffffu, fastm);
+        const unsigned todo = __ballot_sync(0xffffffffu, go), fastb = __ballot_sync(0xffffffffu, fastm) & todo;
         for (int r0 = 0; r0 < 32; r0 += RB) {
-            if (!((todo >> r0) & ((1u << RB) - 1u))) continue;
+            const unsigned fast = (fastb >> r0) & ((1u << RB) - 1u);
+            if (!fast) continue;
             uint64_t pb[RB];
             uint32_t len[RB], col[RB];
             float x[RB], rsi[RB], rinc[RB], aux[RB], acc[RB];
 #pragma unroll
             for (int u = 0; u < RB; ++u) {
                 pb[u] = __shfl_sync(0xffffffffu, pbm, r0 + u);
-                len[u] = __shfl_sync(0xffffffffu, lenm, r0 + u);
+                len[u] = (fast >> u) & 1u ? __shfl_sync(0xffffffffu, lenm, r0 + u) : 0u;
                 rsi[u] = __shfl_sync(0xffffffffu, rc.y, r0 + u);
                 rinc[u] = __shfl_sync(0xffffffffu, rc.z, r0 + u);
                 aux[u] = __shfl_sync(0xffffffffu, rc.w, r0 + u);
@@ -555,23 +558,39 @@ __device__ __forceinline__ void kp_csr_rows(const KmppArgs &a, int first, uint32
             }
 #pragma unroll
             for (int u = 0; u < RB; ++u) {
-                if (!((fastb >> (r0 + u)) & 1u) && ((todo >> (r0 + u)) & 1u)) {
-                    // the pair's own pv: every column with the full scalars
-                    const PairScalars s = pair_scalars(a.prior, a.prior_sum, a.rowsum[g0 + r0 + u], csum, a.d);
-                    float t = 0.f;
-                    for (uint64_t j = lane; j < a.d; j += 32) kp_elem<MSR>(t, raw[j], 0.f, s);
-                    for (uint32_t p = lane; p < len[u]; p += 32) {
-                        const float cj = raw[a.idx[pb[u] + p]];
-                        float t1 = 0.f, t0 = 0.f;
-                        kp_elem<MSR>(t1, cj, a.vals[pb[u] + p], s);
-                        kp_elem<MSR>(t0, cj, 0.f, s);
-                        t = t + (t1 - t0);
-                    }
-                    acc[u] = t;
-                }
 #pragma unroll
                 for (int m = 16; m >= 1; m >>= 1) acc[u] = acc[u] + __shfl_xor_sync(0xffffffffu, acc[u], m);
                 if (lane == r0 + u) accm = acc[u];
+            }
+        }
+        // rows whose pair has a pv of its own (prior 0: nearly all): every column with the full scalars
+        unsigned slow = MSR == SQRL2 ? 0u : todo & ~fastb;
+        if (slow) {
+            PairScalars sm = {0.f, 0.f, 0.f, 0.f, 0.f};
+            if (!fastm) sm = pair_scalars(a.prior, a.prior_sum, a.rowsum[my], csum, a.d);
+            while (slow) {
+                const int r = __ffs(slow) - 1;
+                slow &= slow - 1;
+                PairScalars s;
+                s.pv = __shfl_sync(0xffffffffu, sm.pv, r);
+                s.lhrsi = __shfl_sync(0xffffffffu, sm.lhrsi, r);
+                s.rhrsi = __shfl_sync(0xffffffffu, sm.rhrsi, r);
+                s.lhinc = __shfl_sync(0xffffffffu, sm.lhinc, r);
+                s.rhinc = __shfl_sync(0xffffffffu, sm.rhinc, r);
+                const uint64_t pb = __shfl_sync(0xffffffffu, pbm, r);
+                const uint32_t len = __shfl_sync(0xffffffffu, lenm, r);
+                float t = 0.f;
+                for (uint64_t j = lane; j < a.d; j += 32) kp_elem<MSR>(t, raw[j], 0.f, s);
+                for (uint32_t p = lane; p < len; p += 32) {
+                    const float cj = raw[a.idx[pb + p]];
+                    float t1 = 0.f, t0 = 0.f;
+                    kp_elem<MSR>(t1, cj, a.vals[pb + p], s);
+                    kp_elem<MSR>(t0, cj, 0.f, s);
+                    t = t + (t1 - t0);
+                }
+#pragma unroll
+                for (int m = 16; m >= 1; m >>= 1) t = t + __shfl_xor_sync(0xffffffffu, t, m);
+                if (lane == r) accm = t;
             }
         }
         double v = 0.0;
@@ -1021,7 +1040,7 @@ __global__ void __launch_bounds__(128) k_kmpp_dense_persist(const KmppArgs a, in
 // k_kmpp_csr.
 constexpr uint64_t kKpColsMax = 16384;         // 3 d floats: 192 KB
 constexpr uint64_t kKpPrepMax = 1024ull * 1536;  // d / 32 floats: 192 KB
-constexpr uint64_t kKpCtMax = 49152;           // d floats: 192 KB
+constexpr uint64_t kKpCtMax = 28672;           // d floats: 112 KB, two CTAs per SM
 
 template <int MSR>
 static int kmpp_csr_prepare_t(const KmppArgs &a, float4 *rowc, float *rv, double *brow, int sms, cudaStream_t st) {
@@ -1037,10 +1056,12 @@ int kmpp_csr_prepare(KmppArgs &a, KmppCsrWork &w, uint64_t nnz, int sms, cudaStr
     MC_TRY(w.part.alloc(64, st));
     MC_TRY(w.ticket.alloc(1, st));
     MC_CUDA_TRY(cudaMemsetAsync(w.ticket.p, 0, sizeof(unsigned), st));
-    if (a.msr == JSD) MC_TRY(w.brow.alloc(a.n, st));
+    // the O(nnz) form of JSD alone reads the rows' sums
+    if (a.msr == JSD && a.ct) MC_TRY(w.brow.alloc(a.n, st));
     // the entries' row side pays from a few rounds on; without the memory for it the rounds
-    // form it from the values each time
-    const bool uses = a.msr == MKL || a.msr == HELLINGER || a.msr == JSD;
+    // form it from the values each time.  With prior 0 the pairs have a pv of their own (but where the
+    // rows' sums are not positive) and do not read it
+    const bool uses = (a.msr == MKL || a.msr == HELLINGER || a.msr == JSD) && float(a.prior) > 0.f;
     if (uses && a.k >= 4 && nnz && w.rv.alloc(nnz, st) != MC_OK) cudaGetLastError();
     a.rowc = w.rowc.p;
     a.rv = w.rv.p;
@@ -1100,7 +1121,10 @@ static int update_t(const KmppArgs &a, int first, uint32_t round, int sms, cudaS
             k_kmpp_center_prep<MSR><<<kPrepCtas, 128, psm, st>>>(a, round, self ? 1 : 0), note_launch();
             if (MSR == JSD) k_kmpp_jsd_zcol<<<unsigned((a.ngrp + 7) / 8), 256, 0, st>>>(a), note_launch();
             const unsigned blocks = unsigned(umin64(groups, uint64_t(sms) * 2));
-            if (a.d <= kKpCtMax) {
+            // the center in shared memory where two CTAs fit (5,000 x 40,000 rows of 400 entries, Hellinger, eight
+            // centers: 3.5 ms with one CTA per SM, 2.0 from global memory) and the rows read it: those of prior 0
+            // read the plain row, which wants the L1 (20,000 x 20,000, MKL: 10.1 and 7.4 ms)
+            if (a.d <= kKpCtMax && (MSR == SQRL2 || float(a.prior) > 0.f)) {
                 MC_CUDA_TRY(cudaFuncSetAttribute(k_kmpp_csr_nnz<MSR, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  int(kKpCtMax * sizeof(float))));
                 k_kmpp_csr_nnz<MSR, true><<<blocks, kNnzThreads, a.d * sizeof(float), st>>>(a, first, round), note_launch();
