@@ -119,8 +119,7 @@ static int copy_out(T *dst, const T *src, size_t count, cudaStream_t st) {
 
 // CSR structure check (every kernel relies on it): indptr[0] == 0, nondecreasing,
 // indptr[n] == nnz, column indices < d and strictly increasing within each row.
-// One thread per row: rows of a few entries (5 a row, 80,000 rows: 3.6 us against 30 us with a
-// warp per row).
+// One thread per row, for rows of up to some hundred entries.
 __global__ void __launch_bounds__(256) k_validate_csr_short(const uint64_t *__restrict__ indptr,
                                                             const uint32_t *__restrict__ idx, uint64_t n, uint64_t d,
                                                             uint64_t nnz, int *bad) {
@@ -140,8 +139,9 @@ __global__ void __launch_bounds__(256) k_validate_csr_short(const uint64_t *__re
     }
 }
 
-// One warp per row, lanes over its entries: coalesced (1500 entries a row, 100,000 rows: 0.19 ms
-// against 0.83 ms with a thread per row, whose loads touch 32 rows each).
+// One warp per 32 rows, lanes over a row's entries: coalesced, where a thread per row touches 32 rows per
+// load.  In us, this / a thread per row, rows x entries: 100,000 x 1500: 188 / 633; 50,000 x 300: 57 / 95;
+// 20,000 x 200: 31 / 40; 200,000 x 50: 67 / 34; 80,000 x 20: 36 / 7.
 __global__ void __launch_bounds__(256) k_validate_csr(const uint64_t *__restrict__ indptr,
                                                       const uint32_t *__restrict__ idx, uint64_t n, uint64_t d,
                                                       uint64_t nnz, int *bad) {
@@ -188,7 +188,7 @@ static int validate_csr(const uint64_t *indptr, const uint32_t *idx, uint64_t n,
     DBuf<int> flag;
     MC_TRY(flag.alloc(1, st));
     MC_CUDA_TRY(cudaMemsetAsync(flag.p, 0, sizeof(int), st));
-    if (nnz < 16 * n)
+    if (nnz < 160 * n)
         k_validate_csr_short<<<unsigned((n + 255) / 256), 256, 0, st>>>(indptr, idx, n, d, nnz, flag.p), note_launch();
     else
         k_validate_csr<<<unsigned(umin64((n + 255) / 256, 152 * 8)), 256, 0, st>>>(indptr, idx, n, d, nnz, flag.p),

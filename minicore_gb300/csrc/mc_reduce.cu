@@ -327,83 +327,46 @@ __global__ void k_row_sums_dense(const float *__restrict__ X, uint64_t n, uint64
     if (rownorm) rownorm[i] = q;
 }
 
-// FP64 row sums in entry order, one thread per row: rows of a few entries.
-__global__ void k_row_sums_csr_short(const float *__restrict__ vals, const uint64_t *__restrict__ indptr, uint64_t n,
-                                     double *rowsum) {
+// FP64 row sums in entry order, one thread per row (marked: only the rows that k_row_sums_csr_whole
+// marked as not its own).
+__global__ void __launch_bounds__(128) k_row_sums_csr(const float *__restrict__ vals,
+                                                      const uint64_t *__restrict__ indptr, uint64_t n, int marked,
+                                                      double *rowsum) {
     const uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
     if (i >= n) return;
+    if (marked && (__double_as_longlong(rowsum[i]) & 0x7fffffffffffffffll) <= 0x7ff0000000000000ll) return;
     double s = 0.0;
     for (uint64_t p = indptr[i]; p < indptr[i + 1]; ++p) s = s + double(vals[p]);
     rowsum[i] = s;
 }
 
-// The same, a warp per 32 rows.  Whole-number values (counts) below 2^31
-// are added as integers, lanes over a row's entries: every partial sum is exact, so the order
-// does not matter and the total is the sequential one (rows of fewer than 2^21 entries stay
-// below 2^53).  Rows with any other value are added by their own lane from a 32 x 32 tile in
-// shared memory, entries in order.  1500 entries a row, 100,000 rows: 0.23 ms against 0.70 ms
-// with a thread per row, whose loads touch 32 rows each; 5 entries a row, 80,000 rows: 16 us
-// against 8 us, so short rows keep that form.
-__global__ void __launch_bounds__(128) k_row_sums_csr(const float *__restrict__ vals,
-                                                      const uint64_t *__restrict__ indptr, uint64_t n,
-                                                      double *rowsum) {
-    __shared__ float tile[4][32][33];
-    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+// The same for rows of whole numbers (counts) below 2^31, a warp per row: they are added as integers, so
+// every partial sum is exact, the order does not matter and the total is the sequential one (rows of
+// fewer than 2^21 entries stay below 2^53).  Other rows are marked by a NaN, most of them from their
+// first 32 entries.
+__global__ void __launch_bounds__(256) k_row_sums_csr_whole(const float *__restrict__ vals,
+                                                            const uint64_t *__restrict__ indptr, uint64_t n,
+                                                            double *rowsum) {
+    const int lane = threadIdx.x & 31;
     const uint64_t nw = (gridDim.x * uint64_t(blockDim.x)) >> 5;
-    for (uint64_t g0 = ((blockIdx.x * uint64_t(blockDim.x) + threadIdx.x) >> 5) * 32; g0 < n; g0 += nw * 32) {
-        const uint64_t i = g0 + lane;
-        uint64_t bm = 0, em = 0;
-        if (i < n) {
-            bm = indptr[i];
-            em = indptr[i + 1];
+    for (uint64_t i = (blockIdx.x * uint64_t(blockDim.x) + threadIdx.x) >> 5; i < n; i += nw) {
+        const uint64_t b = indptr[i], e = indptr[i + 1];
+        bool ok = e - b < (1ull << 21);
+        long long s = 0;
+        auto add = [&](float v) {
+            const bool whole = fabsf(v) < 2147483648.f && truncf(v) == v;
+            ok &= whole;
+            s += whole ? (long long)(int(v)) : 0ll;
+        };
+        if (b + lane < e) add(vals[b + lane]);
+        if (__all_sync(0xffffffffu, ok)) {
+#pragma unroll 8
+            for (uint64_t p = b + 32 + lane; p < e; p += 32) add(vals[p]);
         }
-        bool whole = true;
-        long long tot = 0;
-        const int rows = int(umin64(32, n - g0));
-        for (int r = 0; r < rows; ++r) {
-            const uint64_t b = __shfl_sync(0xffffffffu, bm, r), e = __shfl_sync(0xffffffffu, em, r);
-            bool ok = e - b < (1ull << 21);
-            long long s = 0;
-            if (ok)
-#pragma unroll 4
-                for (uint64_t p = b + lane; p < e; p += 32) {
-                    const float v = vals[p];
-                    ok &= fabsf(v) < 2147483648.f && truncf(v) == v;
-                    s += (long long)(ok ? int(v) : 0);
-                }
-            ok = __all_sync(0xffffffffu, ok);
+        ok = __all_sync(0xffffffffu, ok);
 #pragma unroll
-            for (int m = 16; m >= 1; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
-            if (lane == r) {
-                whole = ok;
-                tot = s;
-            }
-        }
-        double sum = double(tot);
-        const unsigned todo = __ballot_sync(0xffffffffu, i < n && !whole);
-        if (todo) {
-            uint64_t longest = ((todo >> lane) & 1u) ? em - bm : 0;
-#pragma unroll
-            for (int m = 16; m >= 1; m >>= 1) {
-                const uint64_t o = __shfl_xor_sync(0xffffffffu, longest, m);
-                longest = o > longest ? o : longest;
-            }
-            double s = 0.0;
-            for (uint64_t c0 = 0; c0 < longest; c0 += 32) {
-                __syncwarp();
-                for (int r = 0; r < 32; ++r) {
-                    const uint64_t b = __shfl_sync(0xffffffffu, bm, r), e = __shfl_sync(0xffffffffu, em, r);
-                    if (((todo >> r) & 1u) && b + c0 + lane < e) tile[wp][r][lane] = vals[b + c0 + lane];
-                }
-                __syncwarp();
-                if ((todo >> lane) & 1u) {
-                    const int cnt = int(em - bm > c0 ? umin64(32, em - bm - c0) : 0);
-                    for (int q = 0; q < cnt; ++q) s = s + double(tile[wp][lane][q]);
-                }
-            }
-            if ((todo >> lane) & 1u) sum = s;
-        }
-        if (i < n) rowsum[i] = sum;
+        for (int m = 16; m >= 1; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
+        if (lane == 0) rowsum[i] = ok ? double(s) : __longlong_as_double(0x7ff8000000000000ll);
     }
 }
 
@@ -467,8 +430,14 @@ int launch_row_sums_dense(const float *X, uint64_t n, uint64_t d, double *rowsum
 int launch_row_sums_csr(const float *vals, const uint64_t *indptr, uint64_t n, uint64_t nnz, double *rowsum,
                         cudaStream_t st) {
     if (n == 0) return MC_OK;
-    auto kern = nnz < 16 * n ? k_row_sums_csr_short : k_row_sums_csr;
-    kern<<<unsigned((n + 127) / 128), 128, 0, st>>>(vals, indptr, n, rowsum), note_launch();
+    // From 512 entries a row on, a warp per row gains more on counts than its first loads cost elsewhere: in us,
+    // with it / a thread per row alone, 100,000 x 1500: 114 / 662 (fractions 680 / 660); 100,000 x 512:
+    // 61 / 232 (247 / 232); 5,000 x 1500: 14 / 155 (158 / 154)
+    const bool wide = nnz >= 512 * n;
+    if (wide)
+        k_row_sums_csr_whole<<<unsigned(umin64((n + 7) / 8, 152 * 16)), 256, 0, st>>>(vals, indptr, n, rowsum),
+            note_launch();
+    k_row_sums_csr<<<unsigned((n + 127) / 128), 128, 0, st>>>(vals, indptr, n, wide ? 1 : 0, rowsum), note_launch();
     MC_CUDA_TRY(cudaGetLastError());
     return MC_OK;
 }
