@@ -1115,11 +1115,11 @@ __global__ void __launch_bounds__(256) k_soft_center_chunks(const float *__restr
         unsigned long long s[2] = {0ull, 0ull}, e[2] = {0ull, 0ull};
 #pragma unroll 4
         for (int r = 0; r < cnt; ++r) {
+            // the products round to float first (a packed product would be fused into the sums)
             const float x = xs[r * 32 + lane];
-            const ulonglong2 cf = *reinterpret_cast<const ulonglong2 *>(co + r * 32 + 4 * wp);
-            const unsigned long long xx = c2_pack(x, x);
-            c2_two_sum_add(s[0], e[0], c2_mul(cf.x, xx));
-            c2_two_sum_add(s[1], e[1], c2_mul(cf.y, xx));
+            const float4 cf = *reinterpret_cast<const float4 *>(co + r * 32 + 4 * wp);
+            c2_two_sum_add(s[0], e[0], c2_pack(__fmul_rn(cf.x, x), __fmul_rn(cf.y, x)));
+            c2_two_sum_add(s[1], e[1], c2_pack(__fmul_rn(cf.z, x), __fmul_rn(cf.w, x)));
         }
         if (jon) {
 #pragma unroll
