@@ -580,6 +580,7 @@ __device__ __forceinline__ void kp_csr_rows(const KmppArgs &a, int first, uint32
                 const uint64_t pb = __shfl_sync(0xffffffffu, pbm, r);
                 const uint32_t len = __shfl_sync(0xffffffffu, lenm, r);
                 float t = 0.f;
+#pragma unroll (MSR == L1 ? 16 : 4)
                 for (uint64_t j = lane; j < a.d; j += 32) kp_elem<MSR>(t, raw[j], 0.f, s);
                 for (uint32_t p = lane; p < len; p += 32) {
                     const float cj = raw[a.idx[pb + p]];
@@ -1134,8 +1135,11 @@ static int update_t(const KmppArgs &a, int first, uint32_t round, int sms, cudaS
         } else if (a.d <= kKpColsMax) {
             MC_CUDA_TRY(cudaFuncSetAttribute(k_kmpp_csr_cols<MSR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              int(kKpColsMax * 12)));
-            k_kmpp_csr_cols<MSR><<<unsigned(umin64((groups + 7) / 8, uint64_t(sms) * 8)), 256, 3 * a.d * sizeof(float),
-                                   st>>>(a, first, round), note_launch();
+            // few rows: a group each on the SMs' CTAs (two while their columns fit) rather than eight on a few SMs
+            // (10,000 x 15,000 rows of 900 entries, JSD of mixed sums, eight centers: 9.0 -> 7.3 ms)
+            const uint64_t spread = umin64(groups, uint64_t(sms) * (a.d <= kKpColsMax / 2 ? 2 : 1)), full = umin64((groups + 7) / 8, uint64_t(sms) * 8);
+            k_kmpp_csr_cols<MSR><<<unsigned(spread > full ? spread : full), 256, 3 * a.d * sizeof(float), st>>>(a, first, round),
+                note_launch();
         } else {
             k_kmpp_csr<MSR><<<unsigned(umin64((a.n + 7) / 8, uint64_t(sms) * 16)), 256, 0, st>>>(a, first, round),
                 note_launch();
