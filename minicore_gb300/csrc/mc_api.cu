@@ -424,8 +424,12 @@ int job_assign_with(mc_job *j, const float *C, double prior_sum, bool force_exac
     }
     if (sparse && j->msr == JSD) {
         MC_TRY(j->ztab.alloc(uint64_t(j->ngrp) * j->k, j->st));
-        MC_TRY(j->jlogs.alloc(2 * uint64_t(jsd_log_centers(j->k, d)) * d, j->st));
-        MC_TRY(launch_jsd_ztable(C, j->k, d, j->csum.p, j->pv, j->gval.p, j->ngrp, j->ztab.p, j->jlogs.p, j->st));
+        float *logs = nullptr;
+        if (jsd_logs_pay(j->ngrp, j->k, d)) {
+            MC_TRY(j->jlogs.alloc(2 * uint64_t(jsd_log_centers(j->k, d)) * d, j->st));
+            logs = j->jlogs.p;
+        }
+        MC_TRY(launch_jsd_ztable(C, j->k, d, j->csum.p, j->pv, j->gval.p, j->ngrp, j->ztab.p, logs, j->st));
         a.grp = j->grp.p;
         a.ztab = j->ztab.p;
     }

@@ -140,9 +140,11 @@ __global__ void __launch_bounds__(256) k_jsd_center_logs(const float *__restrict
     }
 }
 
-__global__ void __launch_bounds__(256) k_jsd_ztable(const float2 *__restrict__ ca, uint32_t kc, uint32_t c0,
-                                                    uint32_t k, uint64_t d, const float *__restrict__ gval,
-                                                    uint32_t ngrp, double *ztab) {
+// RAW: from the centers C (ca then points at them) and their sums, a second logarithm per term
+template <bool RAW>
+__global__ void __launch_bounds__(256) k_jsd_ztable(const float2 *__restrict__ ca, const double *__restrict__ csum,
+                                                    float pv, uint32_t kc, uint32_t c0, uint32_t k, uint64_t d,
+                                                    const float *__restrict__ gval, uint32_t ngrp, double *ztab) {
     const int lane = threadIdx.x & 31;
     const uint64_t wid = (blockIdx.x * uint64_t(blockDim.x) + threadIdx.x) >> 5;
     if (wid >= uint64_t(ngrp) * kc) return;  // whole warp
@@ -150,10 +152,19 @@ __global__ void __launch_bounds__(256) k_jsd_ztable(const float2 *__restrict__ c
     const float b = gval[g];
     const float blb = b * logf(b);
     const float2 *r = ca + uint64_t(c) * d;
+    const float *x = reinterpret_cast<const float *>(ca) + uint64_t(c) * d;
+    float rsi = 0.f, inc = 0.f;
+    if (RAW) side_scalars(pv, csum[c], d, rsi, inc);
     double s = 0.0;
 #pragma unroll 4
     for (uint64_t j = lane; j < d; j += 32) {
-        const float2 v = __ldg(r + j);
+        float2 v;
+        if (RAW) {
+            v.x = __ldg(x + j) * rsi + inc;
+            v.y = v.x * logf(v.x);
+        } else {
+            v = __ldg(r + j);
+        }
         const float m = v.x + b;
         s = s + widen((v.y + blb) - m * logf(m * 0.5f));
     }
@@ -170,6 +181,12 @@ uint32_t jsd_log_centers(uint32_t k, uint64_t d) {
 int launch_jsd_ztable(const float *C, uint32_t k, uint64_t d, const double *csum, float pv, const float *gval,
                       uint32_t ngrp, double *ztab, float *alog, cudaStream_t st) {
     if (ngrp == 0 || k == 0) return MC_OK;
+    if (!alog) {
+        k_jsd_ztable<true><<<unsigned((uint64_t(ngrp) * k + 7) / 8), 256, 0, st>>>(
+            reinterpret_cast<const float2 *>(C), csum, pv, k, 0, k, d, gval, ngrp, ztab), note_launch();
+        MC_CUDA_TRY(cudaGetLastError());
+        return MC_OK;
+    }
     float2 *ca = reinterpret_cast<float2 *>(alog);
     const uint32_t step = jsd_log_centers(k, d);
     for (uint32_t c0 = 0; c0 < k; c0 += step) {
@@ -177,8 +194,8 @@ int launch_jsd_ztable(const float *C, uint32_t k, uint64_t d, const double *csum
         k_jsd_center_logs<<<dim3(unsigned(umin64((d + 255) / 256, 1024)), kc), 256, 0, st>>>(C + uint64_t(c0) * d, d,
                                                                                              csum + c0, pv, ca),
             note_launch();
-        k_jsd_ztable<<<unsigned((uint64_t(ngrp) * kc + 7) / 8), 256, 0, st>>>(ca, kc, c0, k, d, gval, ngrp, ztab),
-            note_launch();
+        k_jsd_ztable<false><<<unsigned((uint64_t(ngrp) * kc + 7) / 8), 256, 0, st>>>(ca, csum, pv, kc, c0, k, d, gval,
+                                                                                     ngrp, ztab), note_launch();
     }
     MC_CUDA_TRY(cudaGetLastError());
     return MC_OK;

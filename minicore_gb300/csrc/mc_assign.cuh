@@ -98,8 +98,11 @@ uint64_t l1_union_work_entries(uint32_t k, uint64_t d);
 constexpr uint64_t kL1UnionMaxEntries = 1ull << 29;
 // JSD sparse-dot table: ztab[g * k + c] = sum over all columns j of f(a_cj, gval[g]) with
 // f(a, b) = a log a + b log b - (a + b) log((a + b) / 2) and a_cj the center transform; alog: 2 d
-// jsd_log_centers() floats of work space (the transform and a log a of that many centers at a time)
+// jsd_log_centers() floats of work space (the transform and a log a of that many centers at a time), or
+// null: every term forms its center's a log a itself, which pays for small tables (jsd_logs_pay)
 uint32_t jsd_log_centers(uint32_t k, uint64_t d);
+// 2,527 x 103, k = 10, 100 groups, an assignment: 47 us with the logarithms in a launch of their own, 42 without
+inline bool jsd_logs_pay(uint64_t ngrp, uint64_t k, uint64_t d) { return ngrp * k * d >= 2000000; }
 int launch_jsd_ztable(const float *C, uint32_t k, uint64_t d, const double *csum, float pv, const float *gval,
                       uint32_t ngrp, double *ztab, float *alog, cudaStream_t st);
 // row / center part of an L1Stat (dense rows; csum: the centers' sums)
