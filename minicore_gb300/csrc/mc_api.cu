@@ -1496,9 +1496,20 @@ static int job_create_impl(mc_context *ctx, const mc_matrix *X, const float *cen
         if (center_ids) MC_TRY(copy_out(center_ids, ids.p, k, st));
         MC_TRY(sync(st));
     }
+    // plain L1 differences (l1_plain): what the rows allow, read back with the sums below where the prior
+    // already makes it pair mode
+    const bool l1_offer = msr == L1 && j->M.kind == MC_DENSE_F32 && l1_dense_pays(n, d, k);
+    L1Stat rows;
+    auto l1_rows = [&]() -> int {
+        MC_TRY(j->l1stat.alloc(1, st));
+        MC_TRY(launch_l1_row_stat(j->M.X, n * d, j->rowsum.p, n, j->l1stat.p, st));
+        MC_CUDA_TRY(cudaMemcpyAsync(&rows, j->l1stat.p, sizeof(rows), cudaMemcpyDeviceToHost, st));
+        return MC_OK;
+    };
     // constant-prior check: pv == prior for every pair when prior >= smallest_pv at the
     // largest row and center sums (centers are means or rows, so bounded by the rows)
     if (msr != SQRL2) {
+        if (l1_offer && !(float(prior) > 0.f)) MC_TRY(l1_rows());
         MC_TRY(launch_center_sums(j->C.p, k, d, j->csum.p, nullptr, st));
         std::vector<double> rs(n), cs(k);
         MC_CUDA_TRY(cudaMemcpyAsync(rs.data(), j->rowsum.p, n * sizeof(double), cudaMemcpyDeviceToHost, st));
@@ -1518,12 +1529,11 @@ static int job_create_impl(mc_context *ctx, const mc_matrix *X, const float *cen
             MC_TRY(launch_row_scalars(j->rowsum.p, n, d, j->pv, j->rsi.p, j->rinc.p, st));
         }
     }
-    if (msr == L1 && j->pair && j->M.kind == MC_DENSE_F32 && l1_dense_pays(n, d, k)) {
-        L1Stat rows;
-        MC_TRY(j->l1stat.alloc(1, st));
-        MC_TRY(launch_l1_row_stat(j->M.X, n * d, j->rowsum.p, n, j->l1stat.p, st));
-        MC_CUDA_TRY(cudaMemcpyAsync(&rows, j->l1stat.p, sizeof(rows), cudaMemcpyDeviceToHost, st));
-        MC_TRY(sync(st));
+    if (l1_offer && j->pair) {
+        if (!j->l1stat.p) {
+            MC_TRY(l1_rows());
+            MC_TRY(sync(st));
+        }
         double xsum;
         float xmin;
         std::memcpy(&xsum, &rows.xsum, sizeof(xsum));

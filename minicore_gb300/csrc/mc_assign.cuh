@@ -26,12 +26,13 @@ __host__ __device__ inline bool l1_plain_bounds(double sums, double prior, float
 // the pair kernel's CTAs that leave cost some 17 us, and below 38,912 rows its 128-row tiles leave SMs
 // idle.  Assignment in us, offered / the pair kernel alone, over the grid named at assign_dense_pays
 // (n x d, k; work: n d times k rounded up to the pair kernel's 32): up to 16 centers, which that kernel
-// pads to 32, it pays from a work of 1.2e8 (300,000 x 20, k = 10: 65 / 95); else from 4e8 and 32 columns
+// pads to 32, it pays from a work of 1.2e8 (300,000 x 20, k = 10: 65 / 95), taken from 2.5e8, where a few
+// passes make up for the 30 us that the rows' bounds take once per job; else from 4e8 and 32 columns
 // (100,000 x 64, k = 50: 92 / 117), below which it loses (60,000 x 32, k = 64, 1.2e8: 64 / 54;
 // 75,000 x 50, k = 32, 1.2e8: 63 / 54; 60,000 x 16, k = 1000, 9.8e8: 406 / 347)
 inline bool l1_dense_pays(uint64_t n, uint64_t d, uint32_t k) {
     const double work = double(n) * double(d) * double((uint64_t(k) + 31) / 32 * 32);
-    return n > 128 * 152 * 2 && (k <= 16 ? work >= 1.2e8 : d >= 32 && work >= 4e8);
+    return n > 128 * 152 * 2 && (k <= 16 ? work >= 2.5e8 : d >= 32 && work >= 4e8);
 }
 
 struct AssignArgs {
