@@ -99,6 +99,9 @@ uint64_t mc_kernel_launches(void);
  * its tensor memory and returns, and the call reports MC_ETIMEOUT; the context stays
  * usable.  One shot: later passes run normally. */
 int mc_test_tc_stall_once(void);
+/* Test hook for the paths that run out of device memory: the nth device allocation that the calling
+ * thread's calls make from now on fails, once (0: none).  made: the allocations made so far, or null. */
+int mc_test_refuse_alloc(uint64_t nth, uint64_t *made);
 /* Measured logf throughput of `device` (logf results per second, full occupancy, 8
  * independent chains per thread): the compute roof against which the CSR JSD sparse dot
  * (two logf per nonzero and center) is reported.  Diagnostics; no reference counterpart. */

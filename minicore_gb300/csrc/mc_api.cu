@@ -31,9 +31,25 @@ void note_launch() {
     g_launches.fetch_add(1, std::memory_order_relaxed);
     ++t_launches;
 }
-static thread_local uint64_t t_allocs = 0;
-void note_device_alloc() { ++t_allocs; }
+static thread_local uint64_t t_allocs = 0, t_refused = 0;  // t_refused: the allocation that the test hook refuses
+bool note_device_alloc() { return ++t_allocs != t_refused; }
 uint64_t device_allocs() { return t_allocs; }
+
+bool device_room_to_spare(uint64_t bytes) {
+    if (bytes <= (uint64_t(8) << 20)) return true;  // not worth the query
+    int dev = 0;
+    size_t free = 0, total = 0;
+    cudaMemPool_t pool = nullptr;
+    uint64_t reserved = 0, used = 0;  // the pool's idle memory is the library's to use
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaMemGetInfo(&free, &total) != cudaSuccess ||
+        cudaDeviceGetDefaultMemPool(&pool, dev) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return free + (reserved - used) >= bytes + total / 16;
+}
 
 static std::atomic<bool> g_prof_on{false};
 static std::mutex g_prof_mu;
@@ -271,6 +287,7 @@ struct mc_job {
     DBuf<float> gval;
     DBuf<double> ztab;
     DBuf<float> jlogs;      // centers' a and a log a
+    bool jlogs_refused = false;
     uint32_t ngrp = 0;
     // rows listed by group, for k_assign_jsd_groups (jgroups: it takes this job's passes of as many
     // centers as pay)
@@ -309,6 +326,18 @@ namespace {
 int sync(cudaStream_t st) {
     MC_CUDA_TRY(cudaStreamSynchronize(st));
     return MC_OK;
+}
+
+// The seeding rounds (rounds(a) runs them from the start).  Where they run out of memory that the entries'
+// row sides (KmppCsrWork::rv) hold, they run again without: the rounds then form them from the values.
+template <class Rounds>
+int kmpp_rounds(KmppArgs &a, KmppCsrWork &cw, const Rounds &rounds) {
+    const int rc = rounds(a);
+    if (rc != MC_ENOMEM || !cw.rv.p) return rc;
+    cudaGetLastError();
+    cw.rv.release();
+    a.rv = nullptr;
+    return rounds(a);
 }
 
 // CSR JSD with a constant prior: the zero entries of row i all take the value
@@ -425,8 +454,10 @@ int job_assign_with(mc_job *j, const float *C, double prior_sum, bool force_exac
     if (sparse && j->msr == JSD) {
         MC_TRY(j->ztab.alloc(uint64_t(j->ngrp) * j->k, j->st));
         float *logs = nullptr;
-        if (jsd_logs_pay(j->ngrp, j->k, d)) {
-            MC_TRY(j->jlogs.alloc(2 * uint64_t(jsd_log_centers(j->k, d)) * d, j->st));
+        if (jsd_logs_pay(j->ngrp, j->k, d) && !j->jlogs_refused) {
+            const int rc = j->jlogs.alloc(2 * uint64_t(jsd_log_centers(j->k, d)) * d, j->st);
+            if (rc != MC_OK) cudaGetLastError();  // no room: the terms form them
+            j->jlogs_refused = rc != MC_OK;       // and no later pass, which may be captured, asks again
             logs = j->jlogs.p;
         }
         MC_TRY(launch_jsd_ztable(C, j->k, d, j->csum.p, j->pv, j->gval.p, j->ngrp, j->ztab.p, logs, j->st));
@@ -1281,6 +1312,11 @@ int mc_test_tc_stall_once(void) {
     tc_stall_next();
     return MC_OK;
 }
+int mc_test_refuse_alloc(uint64_t nth, uint64_t *made) {
+    if (made) *made = t_allocs;
+    t_refused = nth ? t_allocs + nth : 0;
+    return MC_OK;
+}
 
 }  // extern "C"
 
@@ -1490,7 +1526,7 @@ static int job_create_impl(mc_context *ctx, const mc_matrix *X, const float *cen
         a.newc = newc.p;
         KmppCsrWork cw;
         MC_TRY(kmpp_csr_prepare(a, cw, j->M.nnz, ctx->sms, st));
-        MC_TRY(run_kmeanspp(a, u.p, tmp.p, ctx->sms, st));
+        MC_TRY(kmpp_rounds(a, cw, [&](const KmppArgs &b) { return run_kmeanspp(b, u.p, tmp.p, ctx->sms, st); }));
         MC_TRY(launch_gather_rows(j->M.kind == MC_CSR_F32, j->M.X, j->M.vals, j->M.idx, j->M.indptr, d, ids.p, k,
                                   j->C.p, st));
         if (center_ids) MC_TRY(copy_out(center_ids, ids.p, k, st));
@@ -1543,7 +1579,8 @@ static int job_create_impl(mc_context *ctx, const mc_matrix *X, const float *cen
     }
     j->sort.chunk_rows = centroid_chunk_rows(j->M.kind == MC_CSR_F32);
     j->sparse_path = j->M.kind == MC_CSR_F32 && !j->pair && (msr != JSD || j->ngrp > 0);
-    if (j->sparse_path && msr == JSD && jsd_groups_pay(n, d, k, j->M.nnz, j->ngrp)) {
+    // (the lists and the sorts' scratch: about 44 bytes per row)
+    if (j->sparse_path && msr == JSD && jsd_groups_pay(n, d, k, j->M.nnz, j->ngrp) && device_room_to_spare(44 * n)) {
         int rc = jsd_bucket_rows(j->grp.p, n, j->ngrp, j->M.nnz, d, ctx->sms, j->jgw, st);
         if (rc == MC_OK) rc = j->jgw.bx.alloc(n, st);
         if (rc == MC_OK)
@@ -2465,25 +2502,27 @@ static int kmeanspp_impl(mc_context *ctx, const mc_matrix *X, uint32_t k, int ms
     a.newc = newc.p;
     KmppCsrWork cw;
     MC_TRY(kmpp_csr_prepare(a, cw, M.nnz, ctx->sms, st));
-    if (local_trials > 1) MC_TRY(run_kmeanspp_greedy(a, local_trials, seed, tmp.p, ctx->sms, st));
-    else MC_TRY(run_kmeanspp(a, u.p, tmp.p, ctx->sms, st));
-    if (lspp_rounds) MC_TRY(run_lspp(ctx, X, a, k, msr, prior, lspp_rounds, seed, ids.p, asnb.p, dist.p, tmp.p, st));
+    MC_TRY(kmpp_rounds(a, cw, [&](const KmppArgs &b) -> int {
+        if (local_trials > 1) MC_TRY(run_kmeanspp_greedy(b, local_trials, seed, tmp.p, ctx->sms, st));
+        else MC_TRY(run_kmeanspp(b, u.p, tmp.p, ctx->sms, st));
+        if (lspp_rounds) MC_TRY(run_lspp(ctx, X, b, k, msr, prior, lspp_rounds, seed, ids.p, asnb.p, dist.p, tmp.p, st));
+        return MC_OK;
+    }));
     MC_TRY(copy_out(center_ids, ids.p, k, st));
-    DBuf<unsigned char> narrow;
-    DBuf<float> c32;
+    // the row sums are read no more: their 8 bytes per row hold the converted outputs
+    float *c32 = reinterpret_cast<float *>(rowsum.p);
+    unsigned char *narrow = reinterpret_cast<unsigned char *>(c32 + n);
     const unsigned og = unsigned(umin64((n + 255) / 256, uint64_t(ctx->sms) * 8));
     if (asn && asn_bytes < 4) {
-        MC_TRY(narrow.alloc(n * uint64_t(asn_bytes), st));
-        if (asn_bytes == 1) k_narrow_asn<<<og, 256, 0, st>>>(asnb.p, n, narrow.p), note_launch();
-        else k_narrow_asn<<<og, 256, 0, st>>>(asnb.p, n, reinterpret_cast<uint16_t *>(narrow.p)), note_launch();
-        MC_TRY(copy_out(static_cast<unsigned char *>(asn), narrow.p, n * uint64_t(asn_bytes), st));
+        if (asn_bytes == 1) k_narrow_asn<<<og, 256, 0, st>>>(asnb.p, n, narrow), note_launch();
+        else k_narrow_asn<<<og, 256, 0, st>>>(asnb.p, n, reinterpret_cast<uint16_t *>(narrow)), note_launch();
+        MC_TRY(copy_out(static_cast<unsigned char *>(asn), narrow, n * uint64_t(asn_bytes), st));
     } else {
         MC_TRY(copy_out(static_cast<uint32_t *>(asn), asnb.p, n, st));
     }
     if (costs && costs_f32) {
-        MC_TRY(c32.alloc(n, st));
-        k_costs_to_f32<<<og, 256, 0, st>>>(dist.p, n, c32.p), note_launch();
-        MC_TRY(copy_out(static_cast<float *>(costs), c32.p, n, st));
+        k_costs_to_f32<<<og, 256, 0, st>>>(dist.p, n, c32), note_launch();
+        MC_TRY(copy_out(static_cast<float *>(costs), c32, n, st));
     } else {
         MC_TRY(copy_out(static_cast<double *>(costs), dist.p, n, st));
     }

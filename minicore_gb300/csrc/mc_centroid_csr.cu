@@ -384,7 +384,10 @@ int launch_centroid_chunks_csr(const CentroidArgs &a, SortWork &w, uint64_t max_
     if (shift) {
         const uint32_t nb = uint32_t((d + (uint64_t(1) << shift) - 1) >> shift);
         if (!a.keep_bands || !w.bands_ready) {
-            if (w.bands.alloc(n * (uint64_t(nb) + 1), st) != MC_OK) {  // no room for the offsets
+            const uint64_t count = n * (uint64_t(nb) + 1);
+            if (!w.bands_refused && count > w.bands.n)
+                w.bands_refused = !device_room_to_spare(count * sizeof(uint32_t)) || w.bands.alloc(count, st) != MC_OK;
+            if (w.bands_refused) {  // no room for the offsets, which no later update, maybe captured, asks for again
                 cudaGetLastError();
                 *done = false;
                 return MC_OK;

@@ -177,8 +177,8 @@ struct DetInput {
 // device buffers
 // ------------------------------------------------------------------------------------
 // device allocations made through DBuf by the calling thread (a stream capture checks that
-// it made none)
-void note_device_alloc();
+// it made none); false: the test hook refuses this one
+bool note_device_alloc();
 uint64_t device_allocs();
 
 template <class T>
@@ -200,8 +200,8 @@ struct DBuf {
         release();
         st = stream;
         if (count == 0) count = 1;
-        note_device_alloc();
-        cudaError_t e = cudaMallocAsync((void **)&p, count * sizeof(T), stream);
+        cudaError_t e = note_device_alloc() ? cudaMallocAsync((void **)&p, count * sizeof(T), stream)
+                                            : cudaErrorMemoryAllocation;
         if (e != cudaSuccess) {
             p = nullptr;
             return fail(MC_ENOMEM, std::string("device allocation of ") + std::to_string(count * sizeof(T)) +
@@ -211,6 +211,10 @@ struct DBuf {
         return MC_OK;
     }
 };
+
+// Whether buffers of `bytes` that only make a later pass faster, and are kept, may be taken: a sixteenth of
+// the device has to stay free beside them, for what the same job or others must have later.
+bool device_room_to_spare(uint64_t bytes);
 
 // managed memory, or device memory of the current device
 bool is_device_ptr(const void *p);

@@ -21,6 +21,7 @@ struct SortWork {
     uint64_t chunk_rows = 0;      // > 0: a sort also writes chunk_start for chunks of this many rows
     uint64_t chunk_done = 0;      // the chunk rows that chunk_start was last written for by a sort
     bool bands_ready = false;     // bands holds the offsets of the owning job's matrix
+    bool bands_refused = false;   // they did not fit
 };
 
 struct JsdGroupWork {  // rows of a CSR JSD job by bucket
