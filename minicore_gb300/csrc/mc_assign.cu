@@ -56,17 +56,6 @@ __global__ void k_prep_centers(const float *__restrict__ C, uint32_t k, uint32_t
     }
 }
 
-// double(v) by integer operations (a NaN stays one)
-__device__ __forceinline__ double widen(float v) {
-    const unsigned sign = __float_as_uint(v) & 0x80000000u;
-    unsigned b = __float_as_uint(v) & 0x7fffffffu, bias = b >= 0x7f800000u ? 0x70000000u : 0x38000000u;
-    if (b < 0x00800000u) {  // zero or subnormal: 2^24 larger, exponent 24 less
-        b = __float_as_uint(__uint_as_float(b) * 16777216.f);
-        bias = b ? 0x38000000u - (24u << 20) : 0u;
-    }
-    return __hiloint2double(int(sign | ((b >> 3) + bias)), int(b << 29));
-}
-
 // per-center FP64 constants for the sparse-dot kernels.  One warp per center: lane l adds the
 // terms of columns l, l+32, ... (coalesced loads; the logs and square roots in parallel),
 // then the 32 lane partials are added in lane order.  A CTA per warp, as k_center_sums

@@ -138,6 +138,19 @@ __host__ __device__ inline uint64_t det_tmp_size(uint64_t n) {
     return 8 * chunks < 2 * kDetSmemLeaves ? 8 * chunks : 2 * kDetSmemLeaves;
 }
 
+#ifdef __CUDACC__
+// double(v) by integer operations (a NaN stays one): the conversion would take the FP64 pipe
+__device__ __forceinline__ double widen(float v) {
+    const unsigned sign = __float_as_uint(v) & 0x80000000u;
+    unsigned b = __float_as_uint(v) & 0x7fffffffu, bias = b >= 0x7f800000u ? 0x70000000u : 0x38000000u;
+    if (b < 0x00800000u) {  // zero or subnormal: 2^24 larger, exponent 24 less
+        b = __float_as_uint(__uint_as_float(b) * 16777216.f);
+        bias = b ? 0x38000000u - (24u << 20) : 0u;
+    }
+    return __hiloint2double(int(sign | ((b >> 3) + bias)), int(b << 29));
+}
+#endif
+
 // pairwise sum of 32 consecutive elements held one per lane; the result is in lane 0
 __device__ __forceinline__ double lane_pairwise32(double v) {
 #pragma unroll

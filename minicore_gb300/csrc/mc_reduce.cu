@@ -876,7 +876,7 @@ __global__ void __launch_bounds__(128) k_centroid_rows_dense(const float *__rest
         if (WEIGHTED) {
             const double sw = __shfl_sync(0xffffffffu, wt, rel & 31);
 #pragma unroll
-            for (int v = 0; v < V; ++v) acc[v] = fma(sw, double(f[v]), acc[v]);
+            for (int v = 0; v < V; ++v) acc[v] = fma(sw, widen(f[v]), acc[v]);
             if (slice == 0) wq = wq + sw;
         } else if (V == 1) {
             two_sum_add(s1, e1, f[0]);
@@ -1195,8 +1195,11 @@ int launch_centroids(const CentroidArgs &a, SortWork &w, cudaStream_t st, bool p
     if (!a.csr) {
         // the widest columns per lane that still give every lane some
         const uintptr_t xp = reinterpret_cast<uintptr_t>(a.X);
-        if (d >= 96 && d % 4 == 0 && xp % 16 == 0) MC_TRY(centroid_rows_dense<4>(a, w, max_chunks, ch, st));
-        else if (d >= 48 && d % 2 == 0 && xp % 8 == 0) MC_TRY(centroid_rows_dense<2>(a, w, max_chunks, ch, st));
+        // (weighted sums of few chunks: FP64 chains, which more warps share better: 8,443 x 96, k = 2, an update
+        // 224 us with a thread per column, 259 with four columns per lane, 220 so)
+        const bool thin = a.w && max_chunks < 152 * 4;
+        if (!thin && d >= 96 && d % 4 == 0 && xp % 16 == 0) MC_TRY(centroid_rows_dense<4>(a, w, max_chunks, ch, st));
+        else if (!thin && d >= 48 && d % 2 == 0 && xp % 8 == 0) MC_TRY(centroid_rows_dense<2>(a, w, max_chunks, ch, st));
         else MC_TRY(centroid_rows_dense<1>(a, w, max_chunks, ch, st));
     } else {
         bool done = false;
