@@ -1331,11 +1331,20 @@ __global__ void __launch_bounds__(256) k_l1_stat(const float *__restrict__ v, ui
     unsigned mn = 0x7f800000u;
     unsigned long long mx = 0ull;
     const uint64_t i0 = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x, step = gridDim.x * uint64_t(blockDim.x);
-#pragma unroll 4
-    for (uint64_t i = i0; i < m; i += step) {
-        const unsigned b = __float_as_uint(v[i]) & 0x7fffffffu;
+    auto take = [&](float x) {
+        const unsigned b = __float_as_uint(x) & 0x7fffffffu;
         if (b) mn = min(mn, b);  // NaNs are above every finite magnitude
+    };
+    const uint64_t quads = (reinterpret_cast<uintptr_t>(v) & 15) == 0 ? m / 4 : 0;
+#pragma unroll 4
+    for (uint64_t i = i0; i < quads; i += step) {
+        const float4 x = __ldg(reinterpret_cast<const float4 *>(v) + i);
+        take(x.x);
+        take(x.y);
+        take(x.z);
+        take(x.w);
     }
+    for (uint64_t i = 4 * quads + i0; i < m; i += step) take(v[i]);
     for (uint64_t i = i0; i < n; i += step) {
         const double s = sums[i];
         if (!(s <= 0.0)) {
@@ -1359,7 +1368,7 @@ static int l1_stat(const float *v, uint64_t m, const double *sums, uint64_t n, u
                    cudaStream_t st) {
     MC_CUDA_TRY(cudaMemsetAsync(vmin, 0x7f, sizeof(unsigned), st));  // 3.4e38: no nonzero below it
     MC_CUDA_TRY(cudaMemsetAsync(smax, 0, sizeof(unsigned long long), st));
-    k_l1_stat<<<unsigned(umin64((m + 1023) / 1024, 152 * 4)), 256, 0, st>>>(v, m, sums, n, vmin, smax), note_launch();
+    k_l1_stat<<<unsigned(umin64((m + 1023) / 1024, 152 * 8)), 256, 0, st>>>(v, m, sums, n, vmin, smax), note_launch();
     MC_CUDA_TRY(cudaGetLastError());
     return MC_OK;
 }
