@@ -1196,7 +1196,7 @@ int launch_centroids(const CentroidArgs &a, SortWork &w, cudaStream_t st, bool p
         // the widest columns per lane that still give every lane some
         const uintptr_t xp = reinterpret_cast<uintptr_t>(a.X);
         // (weighted sums of few chunks: FP64 chains, which more warps share better: 8,443 x 96, k = 2, an update
-        // 224 us with a thread per column, 259 with four columns per lane, 220 so)
+        // 224 us with a thread per column, 259 with four columns per lane, 200 so)
         const bool thin = a.w && max_chunks < 152 * 4;
         if (!thin && d >= 96 && d % 4 == 0 && xp % 16 == 0) MC_TRY(centroid_rows_dense<4>(a, w, max_chunks, ch, st));
         else if (!thin && d >= 48 && d % 2 == 0 && xp % 8 == 0) MC_TRY(centroid_rows_dense<2>(a, w, max_chunks, ch, st));
