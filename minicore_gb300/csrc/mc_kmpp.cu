@@ -282,9 +282,15 @@ __global__ void __launch_bounds__(256) k_kmpp_csr(const KmppArgs a, int first, u
             s.rhinc = __shfl_sync(0xffffffffu, sm.rhinc, r);
             const uint64_t pb = __shfl_sync(0xffffffffu, pbm, r), pe = __shfl_sync(0xffffffffu, pem, r);
             float acc = 0.f;
-            // (JSD, 20,000 x 20,000, a round: 2.9 ms without the loads of four columns in flight, 1.9 with)
+            // (four columns' loads at a time: JSD, 20,000 x 20,000, a round: 2.9 -> 1.9 ms; with few columns most
+            // lanes have fewer than four: 500,000 x 100, 12 centers: 3.9 ms without, 4.4 with)
+            if (a.d >= 512) {
 #pragma unroll 4
-            for (uint64_t j = lane; j < a.d; j += 32) kp_elem<MSR>(acc, a.cbuf[j], 0.f, s);
+                for (uint64_t j = lane; j < a.d; j += 32) kp_elem<MSR>(acc, a.cbuf[j], 0.f, s);
+            } else {
+#pragma unroll 1
+                for (uint64_t j = lane; j < a.d; j += 32) kp_elem<MSR>(acc, a.cbuf[j], 0.f, s);
+            }
             for (uint64_t p = pb + lane; p < pe; p += 32) {
                 const float cj = a.cbuf[a.idx[p]];
                 float t1 = 0.f, t0 = 0.f;
@@ -1089,7 +1095,14 @@ int kmpp_csr_prepare(KmppArgs &a, KmppCsrWork &w, uint64_t nnz, int sms, cudaStr
 }
 
 static bool kmpp_csr_fused_ok(const KmppArgs &a) { return a.csr && a.msr != JSD && a.ct && a.d <= 4096; }
-static bool kmpp_self_take(const KmppArgs &a) { return a.csr && a.d <= (a.ct ? kKpPrepMax : kKpColsMax); }
+// the column loop beside the center in shared memory; with prior 0, whose rows read the center with scalars of
+// their own, only while few rows leave k_kmpp_csr's higher occupancy unused (12 centers, Hellinger, beside
+// shared memory / k_kmpp_csr: 60,000 x 200 rows of 60 entries 1.45 / 1.60 ms, 206,714 x 194 of 65 4.55 / 3.44,
+// 100,000 x 2,000 of 300 13.8 / 8.7)
+static bool kmpp_csr_cols_ok(const KmppArgs &a) {
+    return a.csr && !a.ct && a.d <= kKpColsMax && (a.msr == SQRL2 || float(a.prior) > 0.f || a.n < 65536);
+}
+static bool kmpp_self_take(const KmppArgs &a) { return a.ct ? a.csr && a.d <= kKpPrepMax : kmpp_csr_cols_ok(a); }
 
 template <int MSR>
 static int update_t(const KmppArgs &a, int first, uint32_t round, int sms, cudaStream_t st) {
@@ -1141,7 +1154,7 @@ static int update_t(const KmppArgs &a, int first, uint32_t round, int sms, cudaS
             } else {
                 k_kmpp_csr_nnz<MSR, false><<<blocks, kNnzThreads, 0, st>>>(a, first, round), note_launch();
             }
-        } else if (a.d <= kKpColsMax) {
+        } else if (kmpp_csr_cols_ok(a)) {
             MC_CUDA_TRY(cudaFuncSetAttribute(k_kmpp_csr_cols<MSR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              int(kKpColsMax * 12)));
             // few rows: a group each on the SMs' CTAs (two while their columns fit) rather than eight on a few SMs

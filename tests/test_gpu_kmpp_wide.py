@@ -68,3 +68,29 @@ def test_wide_rows(n, d, msr, prior):
         assert abs(got - v) <= bound + slack, (i, got, v, bound)
         for w, other in ref:  # the nearest, within the bounds
             assert v - bound <= w + other + slack
+
+
+@pytest.mark.parametrize("msr", [0, 4, 5, 6])
+@pytest.mark.parametrize("n,d", [(65535, 60), (65536, 60), (65600, 600)])
+def test_many_rows_with_prior_zero(n, d, msr):
+    """From 65,536 rows on the column loop with prior 0 is the kernel without shared memory: rows drawn from
+    the whole range, the last one among them, have the bounded distances too."""
+    import minicore_gb300 as mc
+    rng = np.random.default_rng(d + msr)
+    per = 9
+    idx = np.sort(np.argsort(rng.random((n, 40)), axis=1)[:, :per] + rng.integers(0, d - 39, (n, 1)), axis=1)
+    X = sp.csr_matrix((rng.random(n * per).astype(F) * 4 + F(0.25), idx.ravel().astype(np.int32),
+                       np.arange(0, n * per + 1, per)), shape=(n, d))
+    ids, asn, costs = mc.kmeanspp(X, 4, msr=msr, prior=0.0, seed=9)
+    D = np.asarray(X[ids].toarray(), F)
+    for i in [*rng.choice(n, 60).tolist(), n - 1]:
+        if i in ids:
+            assert costs[i] == 0.0
+            continue
+        ref = [_distance(c, np.asarray(X[i].toarray(), F)[0], msr, 0.0) for c in D]
+        got = costs[i] ** 2 * 2 if msr == 6 else costs[i]
+        slack = 2.0 ** -22 * got
+        v, bound = ref[asn[i]]
+        assert abs(got - v) <= bound + slack, (i, got, v, bound)
+        for w, other in ref:
+            assert v - bound <= w + other + slack
