@@ -1375,7 +1375,8 @@ def c4_coreset(args, E):
     obj_full = jfull.cost()
     jfull.close()
     pk, pk_kind = peaks()
-    kmpp_bytes = k * n * d * 4 + k * n * 8 * 2
+    # a round reads the rows' 2-byte copy; the first one, the copy and the row norms read the FP32 rows
+    kmpp_bytes = (k - 1) * n * d * 2 + 3 * n * d * 4 + n * d * 2 + k * n * 8 * 2
     achieved = kmpp_bytes / (stage[0] * 1e-3) / 1e9
     hbm = pk.get("hbm_gbs", 6800.0)
     cpu = None
@@ -1430,7 +1431,7 @@ def c4_coreset(args, E):
             "roofline": {"bound": "hbm", "kernel": "kmeans++ (k passes over the rows)", "achieved": achieved,
                          "peak": hbm, "unit": "GB/s", "frac": achieved / hbm, "traffic": None,
                          "peak_source": f"{pk_kind} hbm_gbs",
-                         "algorithmic": f"k*n*d*4 + 2*k*n*8 = {kmpp_bytes:.4g} bytes"},
+                         "algorithmic": f"(k-1)*n*d*2 + 3*n*d*4 + n*d*2 + 2*k*n*8 = {kmpp_bytes:.4g} bytes"},
             "cpu_baseline": cpu, "gpu_launches": launches, "clocks": clocks, "e2e": e2e}
 
 
