@@ -438,7 +438,8 @@ __device__ __forceinline__ void kp_nnz_term(float &acc, double &bsum, float cj, 
         acc = acc + (m0 * logf(m0 * 0.5f) - m1 * logf(m1 * 0.5f));
     } else {
         // (sqrt a - sqrt b)^2 - (sqrt a - sqrt r)^2 in FP64 from the float roots
-        const double dd = double(cj) - double(v), de = double(cj) - double(aux);
+        // (widened by their bits: three conversions would take the FP64 pipe, which bounds this form)
+        const double dc = widen(cj), dd = dc - widen(v), de = dc - widen(aux);
         bsum = bsum + (dd * dd - de * de);
     }
 }
